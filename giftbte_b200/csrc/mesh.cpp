@@ -408,6 +408,12 @@ Error build_flat_mesh(const RawMesh &raw, const BCs &bcs, const Bands &bands, Fl
                             k1 = q;
                             done[q] = 1;
                             m.cf_face[q] = f;
+                            // one centre per face: the two cells list its
+                            // vertices in different orders, which rounds a
+                            // triangle's mean differently
+                            m.cf_fx[q] = m.cf_fx[k];
+                            m.cf_fy[q] = m.cf_fy[k];
+                            m.cf_fz[q] = m.cf_fz[k];
                         }
                 }
                 m.f_cell0.push_back(c);

@@ -1075,6 +1075,8 @@ __global__ void __launch_bounds__(512) k_residual_tile(DMesh m, DPhys p, EView<S
     }
 }
 
+#include "face_path.cuh"
+
 // One cell of a direction's level order, as the sweep reads it: up to four
 // upwind neighbours (their positions in the same level order, or -(1 +
 // far slot)) with their coefficients a_j = A_f/V (s.n_f) < 0, sig = sum of
@@ -3314,9 +3316,22 @@ Error Solver::init(const FlatMesh &m, const Bands &b, const Angles &a, const std
         bTF_ = up_d(bT);
         bF_dir_ = up_i(dir);
     }
+    // wall slot of every wall face of a cell (-1 on interior faces)
+    {
+        std::vector<int> gw(mesh.ncf(), -1);
+        n_wall_slots_ = 0;
+        for (int k = 0; k < mesh.ncf(); k++)
+            if (mesh.cf_bound[k] >= 0) gw[k] = n_wall_slots_++;
+        cf_gw_ = up_i(gw);
+    }
     if (!ok) return {-6, "device allocation or upload failed"};
     Error e = alloc_all();
     if (e.code) return e;
+    if (mesh.dim == 2)
+        k_face_mask<2><<<grid_for((size_t)nd * mesh.nc), kThreads, 0, s>>>(dm_, dp_, face_mask_);
+    else
+        k_face_mask<3><<<grid_for((size_t)nd * mesh.nc), kThreads, 0, s>>>(dm_, dp_, face_mask_);
+    CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(s));
     initialised = true;
     return {0, ""};
@@ -3381,18 +3396,23 @@ Error Solver::alloc_all() {
     // directions when they fit in 90% of the free device memory, else
     // batches of directions (the intensities, records and schedules stay whole)
     {
-        const size_t per_dir = nc * nb * S * (mesh.dim + 2);
+        // (the gradient buffer also holds the face values of the face-value
+        // path, one row per face; wall_grad_ its gradients at wall faces)
+        const size_t grows = std::max(nc * mesh.dim, (size_t)mesh.nf());
+        const size_t per_dir = nb * S * (grows + 2 * nc + (size_t)n_wall_slots_ * mesh.dim);
         size_t fr = 0, tot = 0;
         CUDA_TRY(cudaMemGetInfo(&fr, &tot));
         const size_t room = fr > (size_t)512 << 20 ? (size_t)((fr - ((size_t)512 << 20)) * 0.9) : 0;
         ndb_ = (int)std::min<size_t>(nd, room / per_dir);
         if (cfg.direction_batch > 0) ndb_ = std::min(ndb_, cfg.direction_batch);
         if (ndb_ < 1) return {-6, "device memory too small for one direction's gradient/residual buffers"};
-        grad_ = A((size_t)ndb_ * nc * nb * mesh.dim * S);
+        grad_ = A((size_t)ndb_ * grows * nb * S);
+        wall_grad_ = A(std::max<size_t>(1, (size_t)ndb_ * n_wall_slots_ * mesh.dim * nb) * S);
+        face_mask_ = (unsigned char *)A(nd * nc);
         res_ = A((size_t)ndb_ * nc * nb * S);
         corr_ = A((size_t)ndb_ * nc * nb * S);
     }
-    for (void *pp : {grad_, res_, corr_, (void *)Tbase_, (void *)Bflux_, (void *)eb_, (void *)cg_scal_})
+    for (void *pp : {grad_, res_, corr_, wall_grad_, (void *)face_mask_, (void *)Tbase_, (void *)Bflux_, (void *)eb_, (void *)cg_scal_})
         if (!pp)
             return {-6, "device allocation failed (" + std::to_string(ne * S * (3 + mesh.dim) / 1048576) +
                             " MiB of band state)"};
@@ -3817,6 +3837,91 @@ Error Solver::cg_solve(const CgPlan &pl, const int *ptr, const int *idx, const d
     return {0, ""};
 }
 
+// lanes per cell and pieces per lane of the face-value gradient
+template <typename S, int DIM>
+constexpr int kFaceW = DIM == 2 && sizeof(S) == 4 ? 4 : 8;
+template <int DIM>
+constexpr int kFaceNP = DIM == 2 ? 2 : 1;
+
+// The face-value path serves the second-order scheme without the limiter
+// when a band row is a whole number of 16-byte pieces; a launch shape fixed
+// by the caller (options.gradient_dirs, residual_form) keeps the
+// gradient-array kernels. FP32 rows of other lengths stay on the one-band
+// kernels, whose face sums are formed in FP64.
+bool Solver::face_path() const {
+    const size_t s = cfg.precision == 1 ? sizeof(float) : sizeof(double);
+    if ((size_t)bands.nb * bands.nmat * 24 > 40 * 1024) return false;  // the band constants are staged per CTA
+    return cfg.order == 2 && !cfg.use_limiter && cfg.gradient_dirs == 0 && cfg.residual_form == 0 &&
+           bands.nb * s % 16 == 0 && (size_t)std::max(mesh.nc, mesh.nf()) * bands.nb < ((size_t)1 << 31);
+}
+
+// Cells per block: 32 in 2D and in the 3D FP32 form, 24 in the 3D FP64 form
+// (two CTAs per SM: its stencil entries are 32 bytes), fewer where a block's
+// tile does not fit in shared memory. Pieces and lanes per cell: 4 lanes of
+// 2 pieces in 2D FP32 and 8 of 2 in 2D FP64 (one stencil entry serves two
+// row loads), 8 of 1 in 3D (a wider slab would leave one CTA per SM).
+template <typename S, int DIM>
+Error Solver::face_shape() {
+    if (fshape_built_) return {0, ""};
+    fshape_built_ = true;
+    cudaStream_t s = cfg.stream;
+    const int best = DIM == 3 && sizeof(S) == 8 ? 24 : 32;
+    for (int B : {best, 16, 8}) {
+        GradTiles t;
+        if (build_grad_tiles(mesh, B, t).code) continue;
+        FaceShape f;
+        f.threads = B * kFaceW<S, DIM>;
+        f.smem = ((size_t)t.qmax + 4 * B) * sizeof(FaceW<S, DIM>) +
+                 (size_t)t.umax * (kFaceW<S, DIM> * kFaceNP<DIM> * 16 + sizeof(int));
+        if (f.smem > 220 * 1024) continue;
+        if (index_checks_enabled()) {
+            long long checked = 0;
+            Error ce = check_tiles(mesh, &t, nullptr, checked);
+            if (ce.code) return ce;
+        }
+        bool ok = true;
+        f.tile.B = t.B, f.tile.nblk = t.nblk, f.tile.umax = t.umax, f.tile.qmax = t.qmax;
+        f.tile.ptr = upload(this, allocs_, t.ptr, s, ok);
+        f.tile.cells = upload(this, allocs_, t.cells, s, ok);
+        f.tile.loc = upload(this, allocs_, t.loc, s, ok);
+        if (!ok) return {-6, "device allocation failed (gradient tiles)"};
+        CUDA_TRY(cudaStreamSynchronize(s));
+        CUDA_TRY(cudaFuncSetAttribute(k_grad_face<S, DIM, kFaceW<S, DIM>, kFaceNP<DIM>>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        fshape_ = f;
+        break;
+    }
+    return {0, ""};
+}
+
+template <typename S, int DIM>
+cudaError_t Solver::launch_grad_face(const S *eps, int d0, int nbt) {
+    constexpr int W = kFaceW<S, DIM>, NP = kFaceNP<DIM>, SW = W * NP;
+    const FaceShape &f = fshape_;
+    const int nb = bands.nb, ppd = nb / kPieceBands<S>;
+    const int slabs = (nbt * ppd + SW - 1) / SW;
+    // slabs per CTA: about eight CTAs for every one that is resident
+    const int per_sm = std::max(1, std::min((int)(227 * 1024 / (f.smem + 1024)), 1024 / f.threads));
+    const int ny = std::max(1, std::min(slabs, (148 * per_sm * 8 + f.tile.nblk - 1) / f.tile.nblk));
+    const int per = (slabs + ny - 1) / ny;
+    const dim3 grid(f.tile.nblk, (slabs + per - 1) / per);
+    k_grad_face<S, DIM, W, NP><<<grid, f.threads, f.smem, cfg.stream>>>(
+        dm_, nb, dm_.lsq_pk, f.tile.ptr, f.tile.cells, f.tile.loc, f.tile.B, f.tile.qmax, f.tile.umax, face_mask_,
+        cf_gw_, n_wall_slots_, eps, (S *)grad_, (S *)wall_grad_, d0, nbt, per);
+    return cudaGetLastError();
+}
+
+template <typename S, int DIM>
+cudaError_t Solver::launch_resid_face(const S *eps, const double *Told, int d0, int nbt) {
+    const int nb = bands.nb, ppd = nb / kPieceBands<S>;
+    const int cpb = std::max(1, std::min(128, 256 / ppd));
+    const dim3 grid((mesh.nc + cpb - 1) / cpb, (nbt + kResDirs - 1) / kResDirs);
+    const size_t smem = (size_t)nb * bands.nmat * (16 + sizeof(S)) + (size_t)kResDirs * cpb * 4 * sizeof(S);
+    k_resid_face<S, DIM><<<grid, ((cpb * ppd + 31) / 32) * 32, smem, cfg.stream>>>(
+        dm_, dp_, cpb, eps, (const S *)grad_, face_mask_, Tbase_, Bflux_, Told, eb_, pos_of_, (S *)res_, d0, nbt);
+    return cudaGetLastError();
+}
+
 template <typename S, int DIM>
 Error Solver::solve_t(SolveStats &st) {
     cudaStream_t s = cfg.stream;
@@ -3973,18 +4078,33 @@ Error Solver::solve_t(SolveStats &st) {
         GL(K_GATHER, k_diffuse_sum<<<grid_for((size_t)nbs * nb), kThreads, 0, s>>>(dm_, dp_, dif_w_, eb_, dsum_));
         GL(K_GATHER, k_gather<<<gB, kThreads, 0, s>>>(dm_, dp_, dsum_, spec_src_, need_snapshot_ ? eb_snap_ : nullptr, eb_));
     };
+    // outgoing wall values of a batch
+    auto bound_out = [&](int d0, int nbt) {
+        const int gr = grid_for((size_t)nbt * nbs * nb);
+        if (face_path() && fshape_.tile.B > 0)
+            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<gr, kThreads, 0, s>>>(dm_, dp_, eps, (const S *)wall_grad_,
+                                                                        n_wall_slots_, cf_gw_, Tbase_, gTb_, eb_, d0,
+                                                                        nbt)));
+        else
+            GL(K_BOUND_OUT, (k_bound_out<S, DIM><<<gr, kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0, nbt)));
+    };
     // LSQ gradient, 4 bands and grad_dg directions per thread (options.gradient_dirs,
     // or timed on the first outer iteration: gtune)
     // (launch shapes: 1, 2, 4 = a thread per cell and 4 bands covering that
     // many directions; 5, 6 = a warp per cell, lanes over band groups and
     // directions, 1 or 2 directions per lane: needs nb / 4 <= 32)
+    if (face_path()) {
+        Error fe = face_shape<S, DIM>();
+        if (fe.code) return fe;
+    }
+    const bool faces = face_path() && fshape_.tile.B > 0;
     const bool wc_ok = nb % 4 == 0 && nb / 4 <= 32;
-    const bool gtune = cfg.gradient_dirs == 0 && tuned_grad_dirs_ == 0 && nb % 4 == 0 && cfg.order == 2;
+    const bool gtune = !faces && cfg.gradient_dirs == 0 && tuned_grad_dirs_ == 0 && nb % 4 == 0 && cfg.order == 2;
     int grad_dg = cfg.gradient_dirs ? cfg.gradient_dirs : tuned_grad_dirs_ ? tuned_grad_dirs_ : 2;
     if (!wc_ok && grad_dg > 4) grad_dg = 2;
     // the tiled form (7, 8: tiles_[0], tiles_[1]): the widest band chunk
     // whose shared memory leaves room for two CTAs per SM, else one
-    if (cfg.order == 2 && nb % 4 == 0) {
+    if (cfg.order == 2 && nb % 4 == 0 && !faces) {
         Error te = grad_tiles();
         if (te.code) return te;
         CUDA_TRY(cudaFuncSetAttribute(k_gradient_tile<S, DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -4104,10 +4224,10 @@ Error Solver::solve_t(SolveStats &st) {
         if (grad_dg >= 9 && (cfg.order != 2 || !tile8_shape(grad_dg, nbc_, thr_, sm_))) grad_dg = 2;
         if (grad_dg >= 7 && grad_dg <= 8 && (cfg.order != 2 || !tile_shape(grad_dg, nbc_, thr_, sm_))) grad_dg = 2;
     }
-    last_grad_dirs_ = nb % 4 == 0 ? grad_dg : 0;
+    last_grad_dirs_ = faces ? 11 : nb % 4 == 0 ? grad_dg : 0;
     // the residual's launch shape (1 = a thread per cell and 4 bands; 5, 6 =
     // a warp per cell as above), timed on the first outer iteration
-    const bool rtune = cfg.residual_form == 0 && tuned_res_form_ == 0 && wc_ok;
+    const bool rtune = !faces && cfg.residual_form == 0 && tuned_res_form_ == 0 && wc_ok;
     int res_form = cfg.residual_form ? cfg.residual_form : tuned_res_form_ ? tuned_res_form_ : 1;
     if (!wc_ok) res_form = 1;
     {
@@ -4140,7 +4260,7 @@ Error Solver::solve_t(SolveStats &st) {
                                                                                       eb_, pos_of_, R, d0, nbt);
         return cudaGetLastError();
     };
-    last_res_form_ = nb % 4 == 0 ? res_form : 0;
+    last_res_form_ = faces ? 9 : nb % 4 == 0 ? res_form : 0;
     // first order (solve_firstorder, StaticBTESyntheticSolver.cpp:487-726):
     // upwind cell values on the faces, i.e. zero gradients throughout
     if (cfg.order == 1) CUDA_TRY(cudaMemsetAsync(grad_, 0, (size_t)ndb * nc * nb * DIM * sizeof(S), s));
@@ -4153,7 +4273,9 @@ Error Solver::solve_t(SolveStats &st) {
             // the gradient in the iteration's launch shape (every shape gives
             // the same bits; the one-band form where bands are not a
             // multiple of 4)
-            if (cfg.order == 2 && nb % 4 == 0)
+            if (faces)
+                GL(K_GRADIENT, CUDA_TRY((launch_grad_face<S, DIM>(eps, d0, nbt))));
+            else if (cfg.order == 2 && nb % 4 == 0)
                 GL(K_GRADIENT, CUDA_TRY(launch_grad(grad_dg, d0, nbt)));
             else if (cfg.order == 2)
                 GL(K_GRADIENT, (k_gradient<S, DIM><<<grid_for((size_t)nbt * nc * nb), kThreads, 0, s>>>(dm_, dp_, w, eps,
@@ -4161,8 +4283,7 @@ Error Solver::solve_t(SolveStats &st) {
             if (cfg.use_limiter)
                 GL(K_GRADIENT, (k_limit<DIM><<<grid_for((size_t)nbt * nc * nb), kThreads, 0, s>>>(
                                    dm_, dp_, (const double *)eps, eb_, (double *)g, d0, nbt)));
-            GL(K_BOUND_OUT, (k_bound_out<S, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev,
-                                                                                                   eb_, d0, nbt)));
+            bound_out(d0, nbt);
         }
         gather();
         CUDA_TRY(cudaGetLastError());
@@ -4192,7 +4313,10 @@ Error Solver::solve_t(SolveStats &st) {
         const int nbt = std::min(ndb, dhi - d0);
         const size_t nbe = (size_t)nbt * nc * nb;
         ev.gd0 = d0;
-        if (nb % 4 == 0) {
+        if (faces) {
+            GL(K_GRADIENT, CUDA_TRY((launch_grad_face<S, DIM>(eps, d0, nbt))));
+            GL(K_RESIDUAL, CUDA_TRY((launch_resid_face<S, DIM>(eps, Told_, d0, nbt))));
+        } else if (nb % 4 == 0) {
             // the residual candidates are timed on the batch's first 16
             // directions when those alone hold millions of (direction, cell)
             // items, enough to fill the GPU; the chosen form then runs on the
@@ -4435,8 +4559,7 @@ Error Solver::solve_t(SolveStats &st) {
         if (dm_.ncross_y > 0)
             GL(K_MOMENTS, (k_cross_cell<S><<<grid_for((size_t)dm_.ncross_y * 32), kThreads, 0, s>>>(
                               dm_, dp_, (const S *)eps, Tbase_, ThC_, QC_, d0, nbt, d0 > dlo ? 1 : 0)));
-        GL(K_BOUND_OUT, (k_bound_out<S, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0,
-                                                                                               nbt)));
+        bound_out(d0, nbt);
         }
         // a shard keeps the boundary values of its own directions only, so
         // that the exchange's sum is their union (x + 0 = x exactly)

@@ -196,6 +196,18 @@ public:
     std::vector<FaceTileDev> ftiles_;  // tiles of the shared-memory residual (residual_form 7, 8)
     bool tiles_built_ = false;
     Error grad_tiles();
+    // the tile and slab shape of the face-value gradient (B = 0: none fits)
+    struct FaceShape {
+        int threads = 0;
+        size_t smem = 0;
+        TileDev tile;
+    };
+    FaceShape fshape_;
+    bool fshape_built_ = false;
+    template <typename S, int DIM> Error face_shape();
+    template <typename S, int DIM> cudaError_t launch_grad_face(const S *eps, int d0, int nbt);
+    template <typename S, int DIM> cudaError_t launch_resid_face(const S *eps, const double *Told, int d0, int nbt);
+    bool face_path() const;
     int tuned_res_form_ = 0;     // residual launch shape (1 thread per cell, 5/6 warp per cell; 0 = not yet tuned)
     int last_res_form_ = 0;      // the same, of the last solve's residual launches (0: 1-band form)
     // launch shape of the last solve's sweep (last_sweep_warp_: 0 block, 1 warp, 2 wide-level kernel)
@@ -223,6 +235,14 @@ private:
     // residuals (level order) and sweep corrections (cell order) for one
     // batch of ndb_ directions [ndb_][nc][nb]
     void *eps_ = nullptr, *grad_ = nullptr, *res_ = nullptr, *corr_ = nullptr;
+    // face-value path: grad_ holds the batch's upwind face values
+    // [ndb_][faces][nb], wall_grad_ its gradients at the wall faces
+    // [ndb_][n_wall_slots_][dim][nb]; face_mask_ [nd][nc] names the faces
+    // each cell writes; cf_gw_ [cell faces] the wall slots
+    void *wall_grad_ = nullptr;
+    unsigned char *face_mask_ = nullptr;
+    int *cf_gw_ = nullptr;
+    int n_wall_slots_ = 0;
     double *Tbase_ = nullptr, *gTb_ = nullptr;
     double *Bflux_ = nullptr;  // [nd][nc] base-field face flux sums of the residual
     double *eb_ = nullptr, *eb_snap_ = nullptr;

@@ -192,13 +192,18 @@ typedef struct {
                                  direction by direction, the rows of the block's stencil union;
                                  9, 10 = the tiles of 7, 8 with eight lanes per cell (FP32-mixed
                                  form, band count a multiple of 32, 40 or 48; others run 2);
-                                 0 = the fastest on the first outer iteration. Results do not
-                                 depend on it. */
+                                 0 = automatic: with residual_form 0 the face-value kernels where
+                                 they apply (second order without the limiter, band rows of whole
+                                 16-byte pieces; gbte_stats.gradient_dirs 11), else the fastest on
+                                 the first outer iteration. Results do not depend on it beyond the
+                                 rounding of the operations after the gradient. */
     int residual_form;        /* launch shape of the second-order residual: 1 = a thread per cell
                                  and 4 bands, 5, 6 = a warp per cell as for gradient_dirs, 7, 8 =
                                  shared-memory tiles of the blocks of gradient_dirs 7, 8 (the
-                                 block's cells and face neighbours); 0 = the fastest on the first
-                                 outer iteration. Results do not depend on it. */
+                                 block's cells and face neighbours); 0 = automatic: with
+                                 gradient_dirs 0 the face-value kernels where they apply
+                                 (gbte_stats.residual_form 9), else the fastest on the first outer
+                                 iteration. Results do not depend on it beyond rounding. */
     int adjoint_history;      /* gbte_vjp: Anderson acceleration of the transposed iteration with
                                  this many difference pairs (1..8); 0 = 6; -1 = the plain iteration
                                  lam += A^-T r. The fixed point, and the stopping rule, are the same. */
