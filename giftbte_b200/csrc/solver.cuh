@@ -123,6 +123,9 @@ struct CgPlan {
     int *part_ptr = nullptr, *perm = nullptr, *ell_col = nullptr, *nsend = nullptr, *snd_src = nullptr,
         *snd_dst = nullptr, *agg_ptr = nullptr;
     double *ell_val = nullptr, *diag = nullptr, *ainv = nullptr;
+    // grid-wide kernel: the whole system in ELL form, column-major
+    int *gcol = nullptr;
+    double *gval = nullptr;
 };
 
 // Sum of `count` doubles of device memory over the handles of a direction
@@ -220,9 +223,11 @@ private:
     Error transient_t(double dt, double total, double err_t, double err_q, int probe, double *hist, long long cap,
                       const std::vector<int> &wall_cell, TransientStats &st);
     Error alloc_all();
-    Error cg_solve(const CgPlan &pl, const int *ptr, const int *idx, const double *val, const double *dinv, double *x,
-                   const double *b, double rtol, double eta, long long &iters, double *scal, double *r, double *z,
-                   double *p, double *Ap, const double *t1, double *sq);
+    Error cg_solve(const CgPlan &pl, const double *dinv, double *x, const double *b, double rtol, double eta,
+                   long long &iters, double *scal, double *r, double *z, double *p, double *Ap, const double *t1,
+                   double *sq);
+    Error ell_plan(const std::vector<int> &ptr, const std::vector<int> &idx, const std::vector<double> &val,
+                   CgPlan &pl);
     Error cg_plan(const std::vector<int> &ptr, const std::vector<int> &idx, const std::vector<double> &val,
                   CgPlan &pl);
     CgPlan kplan_, kfplan_;  // macro and Fourier systems
@@ -276,13 +281,11 @@ private:
     double last_margin_ = 1.0;
     unsigned char *lag_ = nullptr;
     // Fourier pre-solve system (StaticFourier._get_coefficient_macro), negated, CSR
-    int *KF_ptr_ = nullptr, *KF_idx_ = nullptr;
-    double *KF_val_ = nullptr, *KF_dinv_ = nullptr, *bTF_ = nullptr;
+    double *KF_dinv_ = nullptr, *bTF_ = nullptr;
     int *bF_dir_ = nullptr;
     bool fourier_singular_ = true;
     // macro matrix (negated, SPD), CSR
-    int *K_ptr_ = nullptr, *K_idx_ = nullptr;
-    double *K_val_ = nullptr, *K_dinv_ = nullptr;
+    double *K_dinv_ = nullptr;
     double *cg_r_ = nullptr, *cg_z_ = nullptr, *cg_p_ = nullptr, *cg_Ap_ = nullptr, *cg_scal_ = nullptr;
     double *h_pinned_ = nullptr;
     // independent geometries of a batched solve (1 otherwise): cell ranges on

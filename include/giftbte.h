@@ -332,7 +332,7 @@ int gbte_fourier_initial(gbte_handle *h);
  * fragment that pool. Such a caller creates the handle during start-up and
  * re-seeds it here later. The call allocates nothing on the device or in
  * pinned memory. Limits: at most 131072 cells and 131072 node slots (nodes x
- * materials); larger meshes get GBTE_ERR_ARG. The static array (about 7.9 MB)
+ * materials); larger meshes get GBTE_ERR_ARG. The static array (about 7.4 MB)
  * is held by every GPU that loads the library until the process exits. The
  * first call on each device looks up the array's device address and keeps
  * it for the life of that device's primary context (a caller that tears the
