@@ -79,43 +79,68 @@ int grid_for(size_t total, int threads = kThreads) {
     return (int)std::max<size_t>(1, std::min<size_t>(g, 148 * 64));
 }
 
+// a thread per item, kDirShare directions each
+constexpr int kDirShare = 32;
+dim3 dir_grid(size_t items, int nd) {
+    return dim3((unsigned)((items + kThreads - 1) / kThreads), (nd + kDirShare - 1) / kDirShare);
+}
+
 // ---------------------------------------------------------------- kernels --
 
+// The passes that set up the stored deviations and their base. Each owns what
+// does not depend on the direction (a cell's band, a cell's faces) and walks
+// `per` directions of its share, so the cell's index arithmetic, constants
+// and FP64 face geometry are formed once for all of them; bound by the HBM
+// traffic of the band state. 48,000 tetrahedra x 40 bands x 128 directions
+// (FP32), against a thread per value: init 0.64 -> 0.15 ms, rebase 0.77 ->
+// 0.66 ms, face fluxes of the base 0.40 -> 0.04 ms.
+
 template <typename S>
-__global__ void k_init_eps(DMesh m, DPhys p, const double *__restrict__ T0, const double *__restrict__ Tb,
-                           S *__restrict__ eps) {
-    const size_t total = (size_t)p.nd * m.nc * p.nb;
-    for (size_t t = gtid(); t < total; t += gstride()) {
-        int b = (int)(t % p.nb);
-        int c = (int)((t / p.nb) % m.nc);
-        const int mo = mat_off(p, c);
-        eps[t] = (S)(p.C[mo + b] * T0[c] - p.C[mo + b] * Tb[c]);
-    }
+__global__ void __launch_bounds__(256) k_init_eps(DMesh m, DPhys p, const double *__restrict__ T0,
+                                                  const double *__restrict__ Tb, S *__restrict__ eps) {
+    const size_t row = (size_t)m.nc * p.nb, t = gtid();
+    if (t >= row) return;
+    const int b = (int)(t % p.nb), c = (int)(t / p.nb);
+    const int mo = mat_off(p, c);
+    const S v = (S)(p.C[mo + b] * T0[c] - p.C[mo + b] * Tb[c]);
+    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, p.nd);
+    for (int d = blockIdx.y * kDirShare; d < d1; d++) eps[d * row + t] = v;
 }
 
 // eps += C_b (Tb_old - Tb_new): moves the base of the stored deviation to a
 // new per-cell temperature without changing e = C_b Tb + eps
 template <typename S>
-__global__ void k_rebase(DMesh m, DPhys p, const double *__restrict__ Tb_old, const double *__restrict__ Tb_new,
-                         S *__restrict__ eps) {
-    const size_t total = (size_t)p.nd * m.nc * p.nb;
-    for (size_t t = gtid(); t < total; t += gstride()) {
-        const int b = (int)(t % p.nb);
-        const int c = (int)((t / p.nb) % m.nc);
-        eps[t] = (S)((double)eps[t] + p.C[mat_off(p, c) + b] * (Tb_old[c] - Tb_new[c]));
-    }
+__global__ void __launch_bounds__(256) k_rebase(DMesh m, DPhys p, const double *__restrict__ Tb_old,
+                                                const double *__restrict__ Tb_new, S *__restrict__ eps) {
+    const size_t row = (size_t)m.nc * p.nb, t = gtid();
+    if (t >= row) return;
+    const int b = (int)(t % p.nb), c = (int)(t / p.nb);
+    const double Cb = p.C[mat_off(p, c) + b], dT = Tb_old[c] - Tb_new[c];
+    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, p.nd);
+#pragma unroll 8
+    for (int d = blockIdx.y * kDirShare; d < d1; d++) eps[d * row + t] = (S)((double)eps[d * row + t] + Cb * dT);
 }
 
-// least-squares gradient of a cell field with the same stencil
+// least-squares gradient of a cell field with the same stencil. ROUND_EACH:
+// every product rounded before its sum, as the host's compiler does.
+template <bool ROUND_EACH>
 __global__ void k_cell_lsq_grad(DMesh m, const double *__restrict__ T, double *__restrict__ g) {
     const int c = (int)gtid();
     if (c >= m.nc) return;
+    const int q0 = m.nbr_ptr[c], q1 = m.nbr_ptr[c + 1];
+    const double *w = m.lsq_w + 3 * (size_t)q0;
     double gx = 0, gy = 0, gz = 0;
-    for (int q = m.nbr_ptr[c]; q < m.nbr_ptr[c + 1]; q++) {
+    for (int q = q0; q < q1; q++, w += 3) {
         const double de = T[m.nbr_idx[q]] - T[c];
-        gx += m.lsq_w[3 * q] * de;
-        gy += m.lsq_w[3 * q + 1] * de;
-        gz += m.lsq_w[3 * q + 2] * de;
+        if constexpr (ROUND_EACH) {
+            gx = __dadd_rn(gx, __dmul_rn(w[0], de));
+            gy = __dadd_rn(gy, __dmul_rn(w[1], de));
+            gz = __dadd_rn(gz, __dmul_rn(w[2], de));
+        } else {
+            gx += w[0] * de;
+            gy += w[1] * de;
+            gz += w[2] * de;
+        }
     }
     g[3 * c] = gx;
     g[3 * c + 1] = gy;
@@ -546,31 +571,38 @@ __global__ void __launch_bounds__(256) k_gradient_wc(DMesh m, DPhys p, const flo
 template <int DIM>
 __global__ void __launch_bounds__(256) k_base_flux(DMesh m, DPhys p, const double *__restrict__ Tb,
                                                    const double *__restrict__ gTb, double *__restrict__ B) {
-    const int nc = m.nc;
-    const size_t total = (size_t)p.nd * nc;
-    for (size_t t = gtid(); t < total; t += gstride()) {
-        const int c = (int)(t % nc);
-        const size_t d = t / nc;
-        const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
-        const double invV = m.tsc[c] / m.vol[c];
-        double acc = 0;
-        for (int k = m.cf_ptr[c]; k < m.cf_ptr[c + 1]; k++) {
-            const double sn = sx * m.cf_nx[k] + sy * m.cf_ny[k] + (DIM == 3 ? sz * m.cf_nz[k] : 0.0);
-            const double a = m.cf_area[k] * invV * sn;
-            double beta;
-            if (sn >= 0) {
-                beta = Tb[c] + gTb[3 * c] * (m.cf_fx[k] - m.cx[c]) + gTb[3 * c + 1] * (m.cf_fy[k] - m.cy[c]);
-                if (DIM == 3) beta += gTb[3 * c + 2] * (m.cf_fz[k] - m.cz[c]);
-            } else if (m.cf_bound[k] < 0) {
-                const int j = m.cf_nbr[k];
-                beta = Tb[j] + gTb[3 * j] * (m.cf_fx[k] - m.cx[j]) + gTb[3 * j + 1] * (m.cf_fy[k] - m.cy[j]);
-                if (DIM == 3) beta += gTb[3 * j + 2] * (m.cf_fz[k] - m.cz[j]);
-            } else {
-                beta = Tb[c];
-            }
-            acc += a * beta;
+    const int nc = m.nc, c = (int)gtid();
+    if (c >= nc) return;
+    const double invV = m.tsc[c] / m.vol[c];
+    const int k0 = m.cf_ptr[c], nface = m.cf_ptr[c + 1] - k0;
+    // per face: normal, A/V, and the base's face value from either side
+    double nx[4], ny[4], nz[4], av[4], out[4], in[4];
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+        if (f >= nface) continue;
+        const int k = k0 + f;
+        nx[f] = m.cf_nx[k], ny[f] = m.cf_ny[k], nz[f] = DIM == 3 ? m.cf_nz[k] : 0.0;
+        av[f] = m.cf_area[k] * invV;
+        out[f] = Tb[c] + gTb[3 * c] * (m.cf_fx[k] - m.cx[c]) + gTb[3 * c + 1] * (m.cf_fy[k] - m.cy[c]);
+        if (DIM == 3) out[f] += gTb[3 * c + 2] * (m.cf_fz[k] - m.cz[c]);
+        in[f] = Tb[c];
+        if (m.cf_bound[k] < 0) {
+            const int j = m.cf_nbr[k];
+            in[f] = Tb[j] + gTb[3 * j] * (m.cf_fx[k] - m.cx[j]) + gTb[3 * j + 1] * (m.cf_fy[k] - m.cy[j]);
+            if (DIM == 3) in[f] += gTb[3 * j + 2] * (m.cf_fz[k] - m.cz[j]);
         }
-        B[t] = acc;
+    }
+    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, p.nd);
+    for (int d = blockIdx.y * kDirShare; d < d1; d++) {
+        const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
+        double acc = 0;
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+            if (f >= nface) continue;
+            const double sn = sx * nx[f] + sy * ny[f] + (DIM == 3 ? sz * nz[f] : 0.0);
+            acc += av[f] * sn * (sn >= 0 ? out[f] : in[f]);
+        }
+        B[(size_t)d * nc + c] = acc;
     }
 }
 
@@ -3716,16 +3748,15 @@ Error Solver::set_initial(const double *T0, const double *q0, const double *bth)
     }
     // base of the stored deviation: T0 in the FP32 form, 0 in the FP64 form
     if (cfg.precision == 1) {
-        CUDA_TRY(cudaMemcpyAsync(Tbase_, T0, nc * 8, cudaMemcpyHostToDevice, s));
-        // gradient of the base with the same stencil (host, FP64); zero in
-        // the first-order form
-        std::vector<double> g(nc * 3, 0.0);
-        for (size_t c = 0; c < (cfg.order == 2 ? nc : 0); c++)
-            for (int q = mesh.nbr_ptr[c]; q < mesh.nbr_ptr[c + 1]; q++) {
-                double de = T0[mesh.nbr_idx[q]] - T0[c];
-                for (int r = 0; r < 3; r++) g[3 * c + r] += mesh.lsq_w[3 * (size_t)q + r] * de;
-            }
-        CUDA_TRY(cudaMemcpyAsync(gTb_, g.data(), nc * 3 * 8, cudaMemcpyHostToDevice, s));
+        CUDA_TRY(cudaMemcpyAsync(Tbase_, T_, nc * 8, cudaMemcpyDeviceToDevice, s));
+        // gradient of the base with the same stencil; zero in the first-order
+        // form (on the host, one thread, it was 38 of 430 ms of a six-iteration
+        // call on 192,000 tetrahedra)
+        if (cfg.order == 2)
+            k_cell_lsq_grad<true><<<(unsigned)((nc + kThreads - 1) / kThreads), kThreads, 0, s>>>(dm_, Tbase_, gTb_);
+        else
+            CUDA_TRY(cudaMemsetAsync(gTb_, 0, nc * 3 * 8, s));
+        CUDA_TRY(cudaGetLastError());
         CUDA_TRY(cudaStreamSynchronize(s));
     } else {
         CUDA_TRY(cudaMemsetAsync(Tbase_, 0, nc * 8, s));
@@ -4225,11 +4256,9 @@ template <typename S, int DIM>
 Error Solver::solve_t(SolveStats &st) {
     cudaStream_t s = cfg.stream;
     const int nc = mesh.nc, nb = bands.nb, nd = ang.nd, nbs = mesh.nbs(), nslot = mesh.nn * mesh.nmat;
-    const size_t ne = (size_t)nd * nc * nb;
     S *eps = (S *)eps_, *g = (S *)grad_, *R = (S *)res_;
     const S *w = std::is_same<S, float>::value ? (const S *)dm_.lsq_wf : (const S *)dm_.lsq_w;
     EView<S, DIM> ev{eps, g, Tbase_, gTb_, nb, nc, 0};
-    const int gE = grid_for(ne);
     // direction batches: the gradient, residual and correction buffers hold
     // ndb_ directions (all of them when they fit in device memory)
     const int ndb = ndb_;
@@ -4237,7 +4266,6 @@ Error Solver::solve_t(SolveStats &st) {
     const int dlo = dlo_, dhi = dhi_ < 0 ? nd : dhi_;
     const bool sharded = xfn_ != nullptr;
     const int gB = grid_for((size_t)nd * nbs * nb);
-    (void)gE;
     const int gC = (nc + kThreads - 1) / kThreads, gN = (nslot + kThreads - 1) / kThreads;
     // blocks per geometry of the per-geometry reductions
     const int comp_blocks = std::max(1, std::min(148, (nc / ncomp_ + kThreads - 1) / kThreads));
@@ -4565,7 +4593,7 @@ Error Solver::solve_t(SolveStats &st) {
     if (cfg.order == 1) CUDA_TRY(cudaMemsetAsync(grad_, 0, (size_t)ndb * nc * nb * DIM * sizeof(S), s));
     if (!started_) {
         // _set_initial (:765-782) and the initial boundary values (StaticBTESyntheticSolver.cpp:45-62)
-        GL(K_INIT, k_init_eps<S><<<grid_for(ne), kThreads, 0, s>>>(dm_, dp_, T_, Tbase_, eps));
+        GL(K_INIT, k_init_eps<S><<<dir_grid((size_t)nc * nb, nd), kThreads, 0, s>>>(dm_, dp_, T_, Tbase_, eps));
         for (int d0 = 0; d0 < nd; d0 += ndb) {
             const int nbt = std::min(ndb, nd - d0);
             ev.gd0 = d0;
@@ -4589,7 +4617,7 @@ Error Solver::solve_t(SolveStats &st) {
         started_ = true;
     }
     // base-field face fluxes for the current T_base (zero base in FP64)
-    GL(K_INIT, (k_base_flux<DIM><<<grid_for((size_t)nd * nc), kThreads, 0, s>>>(dm_, dp_, Tbase_, gTb_, Bflux_)));
+    GL(K_INIT, (k_base_flux<DIM><<<dir_grid(nc, nd), kThreads, 0, s>>>(dm_, dp_, Tbase_, gTb_, Bflux_)));
     double errOld = 0, errOldq = 0;
     int errInc = 0;
     st = SolveStats();
@@ -5048,13 +5076,12 @@ Error Solver::solve_t(SolveStats &st) {
             if ((it1 & (it1 - 1)) == 0 || it1 % 16 == 0) {
                 GL(K_INIT, k_copy<<<gC, kThreads, 0, s>>>(Tbase_, T1_, nc));
                 GL(K_INIT, k_copy<<<gC, kThreads, 0, s>>>(T_, Tbase_, nc));
-                GL(K_INIT, k_rebase<S><<<gE, kThreads, 0, s>>>(dm_, dp_, T1_, Tbase_, eps));
+                GL(K_INIT, k_rebase<S><<<dir_grid((size_t)nc * nb, nd), kThreads, 0, s>>>(dm_, dp_, T1_, Tbase_, eps));
                 if (cfg.order == 2)
-                    GL(K_INIT, k_cell_lsq_grad<<<gC, kThreads, 0, s>>>(dm_, Tbase_, gTb_));
+                    GL(K_INIT, k_cell_lsq_grad<false><<<gC, kThreads, 0, s>>>(dm_, Tbase_, gTb_));
                 else
                     CUDA_TRY(cudaMemsetAsync(gTb_, 0, (size_t)nc * 3 * 8, s));
-                GL(K_INIT, (k_base_flux<DIM><<<grid_for((size_t)nd * nc), kThreads, 0, s>>>(dm_, dp_, Tbase_, gTb_,
-                                                                                            Bflux_)));
+                GL(K_INIT, (k_base_flux<DIM><<<dir_grid(nc, nd), kThreads, 0, s>>>(dm_, dp_, Tbase_, gTb_, Bflux_)));
             }
         }
         if (errInc >= 10) {
@@ -5112,7 +5139,7 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
     CUDA_TRY(cudaMemsetAsync(q_, 0, (size_t)nc * 24, s));
     CUDA_TRY(cudaMemsetAsync(Tbase_, 0, (size_t)nc * 8, s));
     CUDA_TRY(cudaMemsetAsync(gTb_, 0, (size_t)nc * 24, s));
-    k_init_eps<double><<<grid_for(ne), kThreads, 0, s>>>(dm_, dp_, T_, Tbase_, eps);
+    k_init_eps<double><<<dir_grid((size_t)nc * nb, nd), kThreads, 0, s>>>(dm_, dp_, T_, Tbase_, eps);
     const double *w = dm_.lsq_w;
     const int gB = grid_for((size_t)nd * nbs * nb);
     auto gather = [&]() {
@@ -5397,7 +5424,7 @@ Error Solver::fourier_initial_noalloc() {
     if (cfg.precision == 1) {
         CUDA_TRY(cudaMemcpyAsync(Tbase_, T_, (size_t)nc * sizeof(double), cudaMemcpyDeviceToDevice, s));
         if (cfg.order == 2)
-            GL(K_INIT, k_cell_lsq_grad<<<gC, kThreads, 0, s>>>(dm_, Tbase_, gTb_));
+            GL(K_INIT, k_cell_lsq_grad<false><<<gC, kThreads, 0, s>>>(dm_, Tbase_, gTb_));
         else
             CUDA_TRY(cudaMemsetAsync(gTb_, 0, (size_t)nc * 3 * 8, s));
     } else {
