@@ -405,30 +405,31 @@ __global__ void __launch_bounds__(256, 3) k_resid_face(DMesh m, DPhys p, int cpb
 }
 
 // k_bound_out with the gradients of the wall cells only (gw of k_grad_face):
-// e_c(new) + g_c(pre-sweep) . (x_f - x_c) on the walls a direction leaves
+// e_c(new) + g_c(pre-sweep) . (x_f - x_c) on the walls a direction leaves. A
+// thread per (wall slot, band) walks kDirShare directions: 0.30 -> 0.14 ms
+// against a thread per value (4,800 wall faces x 40 bands x 128 directions).
 template <typename S, int DIM>
-__global__ void k_bound_out_w(DMesh m, DPhys p, const S *__restrict__ eps, const S *__restrict__ gw, int nws,
-                              const int *__restrict__ cf_gw, const double *__restrict__ Tb,
-                              const double *__restrict__ gTb, double *__restrict__ eb, int d0, int ndb) {
-    const int nb = p.nb;
-    const size_t total = (size_t)ndb * m.nbs * nb;
-    for (size_t tl = gtid(); tl < total; tl += gstride()) {
-        const size_t t = tl + (size_t)d0 * m.nbs * nb;  // index over all directions
-        const int b = (int)(tl % nb);
-        const int s = (int)((tl / nb) % m.nbs);
-        const size_t dl = tl / ((size_t)nb * m.nbs), d = d0 + dl;
-        const int c = m.bs_cell[s];
-        if (c < 0) continue;
-        const int k = m.bs_cf[s], mo = mat_off(p, c);
-        const double vm = p.vmag[mo + b];
-        const double vn = vm * p.sx[d] * m.cf_nx[k] + vm * p.sy[d] * m.cf_ny[k] + vm * p.sz[d] * m.cf_nz[k];
-        if (vn >= 0) {
-            const double Cb = p.C[mo + b];
-            const S *gp = gw + (dl * nws + cf_gw[k]) * DIM * nb + b;
-            double v = ((double)gp[0] + Cb * gTb[3 * c]) * (m.cf_fx[k] - m.cx[c]) +
-                       ((double)gp[nb] + Cb * gTb[3 * c + 1]) * (m.cf_fy[k] - m.cy[c]);
-            if (DIM == 3) v += ((double)gp[2 * nb] + Cb * gTb[3 * c + 2]) * (m.cf_fz[k] - m.cz[c]);
-            eb[t] = Cb * Tb[c] + (double)eps[(d * m.nc + c) * nb + b] + v;
-        }
+__global__ void __launch_bounds__(256) k_bound_out_w(DMesh m, DPhys p, const S *__restrict__ eps,
+                                                     const S *__restrict__ gw, int nws,
+                                                     const int *__restrict__ wall_side,
+                                                     const double *__restrict__ Tb, const double *__restrict__ gTb,
+                                                     double *__restrict__ eb, int d0, int ndb) {
+    const int nb = p.nb, t = (int)gtid();
+    if (t >= nws * nb) return;
+    const int w = t / nb, b = t - w * nb, s = wall_side[w], c = m.bs_cell[s], k = m.bs_cf[s], mo = mat_off(p, c);
+    const double vm = p.vmag[mo + b], Cb = p.C[mo + b], Tc = Tb[c];
+    const double nx = m.cf_nx[k], ny = m.cf_ny[k], nz = m.cf_nz[k];
+    const double rx = m.cf_fx[k] - m.cx[c], ry = m.cf_fy[k] - m.cy[c], rz = m.cf_fz[k] - m.cz[c];
+    const double gx = gTb[3 * c], gy = gTb[3 * c + 1], gz = gTb[3 * c + 2];
+    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, ndb);
+#pragma unroll 4
+    for (int dl = blockIdx.y * kDirShare; dl < d1; dl++) {
+        const int d = d0 + dl;
+        const double vn = vm * p.sx[d] * nx + vm * p.sy[d] * ny + vm * p.sz[d] * nz;
+        if (!(vn >= 0)) continue;
+        const S *gp = gw + ((size_t)dl * nws + w) * DIM * nb + b;
+        double v = ((double)gp[0] + Cb * gx) * rx + ((double)gp[nb] + Cb * gy) * ry;
+        if (DIM == 3) v += ((double)gp[2 * nb] + Cb * gz) * rz;
+        eb[((size_t)d * m.nbs + s) * nb + b] = Cb * Tc + (double)eps[((size_t)d * m.nc + c) * nb + b] + v;
     }
 }

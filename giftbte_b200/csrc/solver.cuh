@@ -211,6 +211,7 @@ public:
     template <typename S, int DIM> cudaError_t launch_grad_face(const S *eps, int d0, int nbt);
     template <typename S, int DIM> cudaError_t launch_resid_face(const S *eps, const double *Told, int d0, int nbt);
     bool face_path() const;
+    void launch_walls(bool moments);
     int tuned_res_form_ = 0;     // residual launch shape (1 thread per cell, 5/6 warp per cell; 0 = not yet tuned)
     int last_res_form_ = 0;      // the same, of the last solve's residual launches (0: 1-band form)
     // launch shape of the last solve's sweep (last_sweep_warp_: 0 block, 1 warp, 2 wide-level kernel)
@@ -247,6 +248,7 @@ private:
     void *wall_grad_ = nullptr;
     unsigned char *face_mask_ = nullptr;
     int *cf_gw_ = nullptr;
+    int *wall_side_ = nullptr;  // [n_wall_slots_] boundary side of every wall slot
     int n_wall_slots_ = 0;
     double *Tbase_ = nullptr, *gTb_ = nullptr;
     double *Bflux_ = nullptr;  // [nd][nc] base-field face flux sums of the residual
