@@ -212,6 +212,8 @@ public:
     template <typename S, int DIM> cudaError_t launch_resid_face(const S *eps, const double *Told, int d0, int nbt);
     bool face_path() const;
     void launch_walls(bool moments);
+    size_t moments_smem() const;
+    template <typename S> void launch_moments(S *eps, bool apply, int d0, int nbt, bool accumulate);
     int tuned_res_form_ = 0;     // residual launch shape (1 thread per cell, 5/6 warp per cell; 0 = not yet tuned)
     int last_res_form_ = 0;      // the same, of the last solve's residual launches (0: 1-band form)
     // launch shape of the last solve's sweep (last_sweep_warp_: 0 block, 1 warp, 2 wide-level kernel)
