@@ -301,6 +301,7 @@ private:
     double *h_comp_ = nullptr;
     bool have_initial_ = false;
     bool started_ = false;
+    bool base_is_T_ = false;  // T_ is the base of the deviation (an FP32 start), so the deviation is zero
     int coop_blocks_ = 0;
     cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
     // per-launch profiling (options.profile)
