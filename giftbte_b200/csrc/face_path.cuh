@@ -404,10 +404,95 @@ __global__ void __launch_bounds__(256, 3) k_resid_face(DMesh m, DPhys p, int cpb
     }
 }
 
+// The explicit time step (FP64, base 0) from the face values, in place:
+// e <- e (1 - dt/tau) - dt (sum_f A/V (v.n) x_f - C Told/tau). A thread keeps
+// a 16-byte piece of a cell's bands over kResDirs directions, as k_resid_face
+// does; only the thread that writes a value reads it, so the new field needs
+// no second array and no copy back. Bound by the face rows it streams.
+// 4,608 triangles x 20 bands x 32 directions (FP64): 27 us, and a whole step
+// 287 -> 159 us against gradient arrays, a thread per value and a copy back.
+template <int DIM>
+__global__ void __launch_bounds__(256, 3) k_tr_step_face(DMesh m, DPhys p, int cpb, double *eps,
+                                                         const double *__restrict__ F,
+                                                         const unsigned char *__restrict__ mask,
+                                                         const double *__restrict__ Told,
+                                                         const double *__restrict__ eb, double dt, int d0, int ndb) {
+    constexpr int VE = kPieceBands<double>;
+    extern __shared__ __align__(16) unsigned char rfm[];
+    double *coef = reinterpret_cast<double *>(rfm);  // [kResDirs][cpb][4]
+    const int nb = p.nb, nc = m.nc, nf = m.nf, ppd = nb / VE;
+    const int cb = blockIdx.x * cpb, ncell = min(cpb, nc - cb);
+    const int da = blockIdx.y * kResDirs, nd = min(kResDirs, ndb - da);
+    const int tid = threadIdx.x;
+    for (int t = tid; t < kResDirs * cpb * 4; t += blockDim.x) {
+        const int j = t & 3, ci = (t >> 2) % cpb, dd = (t >> 2) / cpb;
+        double a = 0;
+        if (ci < ncell && dd < nd) {
+            const int c = cb + ci, k = m.cf_ptr[c] + j;
+            if (k < m.cf_ptr[c + 1]) {
+                const size_t d = d0 + da + dd;
+                const double sn = p.sx[d] * m.cf_nx[k] + p.sy[d] * m.cf_ny[k] + (DIM == 3 ? p.sz[d] * m.cf_nz[k] : 0.0);
+                a = m.cf_area[k] / m.vol[c] * sn;
+            }
+        }
+        coef[t] = a;
+    }
+    __syncthreads();
+    const int ci = tid / ppd, b0 = (tid - ci * ppd) * VE;
+    if (ci >= ncell) return;
+    const int c = cb + ci, mo = mat_off(p, c), k0 = m.cf_ptr[c], nface = m.cf_ptr[c + 1] - k0;
+    double keep[VE], src[VE], vm[VE];
+#pragma unroll
+    for (int v = 0; v < VE; v++) {
+        const double tau = p.tau[mo + b0 + v] * m.tsc[c];
+        keep[v] = 1 - dt / tau;
+        src[v] = Told[c] * p.C[mo + b0 + v] / tau;
+        vm[v] = p.vmag[mo + b0 + v];
+    }
+    int at[4];
+    unsigned walls = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        at[j] = j < nface ? m.cf_face[k0 + j] * nb : 0;
+        if (j < nface && m.cf_bound[k0 + j] >= 0) walls |= 1u << j;
+    }
+    double *ep = eps + ((size_t)(d0 + da) * nc + c) * nb + b0;
+    const double *Fp = F + (size_t)da * nf * nb + b0;
+    size_t dc = (size_t)(d0 + da) * nc + c;
+    for (int dd = 0; dd < nd; dd++, dc += nc, ep += (size_t)nc * nb, Fp += (size_t)nf * nb) {
+        double ec[VE], y[4][VE], acc[VE];
+        ld_piece(ep, ec);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (j < nface) ld_piece(Fp + at[j], y[j]);
+        if (walls) {
+            // inflow wall faces take the wall value
+            const unsigned in = walls & ~(unsigned)mask[dc];
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (in >> j & 1)
+                    ld_piece(eb + ((size_t)(d0 + da + dd) * m.nbs + m.cf_bside[k0 + j]) * nb + b0, y[j]);
+        }
+#pragma unroll
+        for (int v = 0; v < VE; v++) acc[v] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (j < nface) {
+                const double a = coef[(dd * cpb + ci) * 4 + j];
+#pragma unroll
+                for (int v = 0; v < VE; v++) acc[v] += a * y[j][v];
+            }
+#pragma unroll
+        for (int v = 0; v < VE; v++) ec[v] = ec[v] * keep[v] - dt * (vm[v] * acc[v] - src[v]);
+        st_piece(ep, ec);
+    }
+}
+
 // k_bound_out with the gradients of the wall cells only (gw of k_grad_face):
 // e_c(new) + g_c(pre-sweep) . (x_f - x_c) on the walls a direction leaves. A
-// thread per (wall slot, band) walks kDirShare directions: 0.30 -> 0.14 ms
-// against a thread per value (4,800 wall faces x 40 bands x 128 directions).
+// thread per (wall slot, band) walks its block's share of the directions
+// (wall_grid): 0.30 -> 0.14 ms against a thread per value (4,800 wall faces x
+// 40 bands x 128 directions).
 template <typename S, int DIM>
 __global__ void __launch_bounds__(256) k_bound_out_w(DMesh m, DPhys p, const S *__restrict__ eps,
                                                      const S *__restrict__ gw, int nws,
@@ -421,9 +506,9 @@ __global__ void __launch_bounds__(256) k_bound_out_w(DMesh m, DPhys p, const S *
     const double nx = m.cf_nx[k], ny = m.cf_ny[k], nz = m.cf_nz[k];
     const double rx = m.cf_fx[k] - m.cx[c], ry = m.cf_fy[k] - m.cy[c], rz = m.cf_fz[k] - m.cz[c];
     const double gx = gTb[3 * c], gy = gTb[3 * c + 1], gz = gTb[3 * c + 2];
-    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, ndb);
+    const int per = (ndb + gridDim.y - 1) / gridDim.y, d1 = min((int)(blockIdx.y + 1) * per, ndb);
 #pragma unroll 4
-    for (int dl = blockIdx.y * kDirShare; dl < d1; dl++) {
+    for (int dl = blockIdx.y * per; dl < d1; dl++) {
         const int d = d0 + dl;
         const double vn = vm * p.sx[d] * nx + vm * p.sy[d] * ny + vm * p.sz[d] * nz;
         if (!(vn >= 0)) continue;

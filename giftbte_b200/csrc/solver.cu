@@ -84,6 +84,14 @@ constexpr int kDirShare = 32;
 dim3 dir_grid(size_t items, int nd) {
     return dim3((unsigned)((items + kThreads - 1) / kThreads), (nd + kDirShare - 1) / kDirShare);
 }
+// the same with as few directions per thread (2 at least) as it takes to give
+// every SM four blocks; the kernel takes its share from the grid (240 wall
+// faces x 20 bands x 32 directions: one thread for all of them 19.4 us, now 6.9)
+dim3 wall_grid(size_t items, int nd) {
+    const int gx = (int)((items + kThreads - 1) / kThreads);
+    const int want = std::max((nd + kDirShare - 1) / kDirShare, (4 * 148 + gx - 1) / gx);
+    return dim3(gx, std::min(want, (nd + 1) / 2));
+}
 
 // ---------------------------------------------------------------- kernels --
 
@@ -1949,7 +1957,12 @@ __global__ void k_remacro(DMesh m, const double *__restrict__ Th, const double *
 // formed once per thread, where four kernels with a thread per (direction,
 // side, band) or a warp per side formed them per value, divisions included:
 // 4,800 wall faces x 40 bands x 128 directions 0.79 -> 0.25 ms.
-constexpr int kWallSlots = 8;
+// With few walls it is bound by the latency of its own chain over the
+// directions: the second pass loads kWallBatch values before it stores any
+// (the compiler cannot move a load over the stores to eb), and blocks hold
+// fewer walls so that every SM has one (launch_walls): the refresh of 240 wall
+// faces x 20 bands x 32 directions 30 -> 19 us.
+constexpr int kWallSlots = 8, kWallBatch = 8;
 template <bool MOM>
 __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nws, const int *__restrict__ wall_side,
                                                const double *__restrict__ wtab, const double *__restrict__ dif_w,
@@ -1977,8 +1990,9 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
         const bool dif = type == 2 || type == 6;
         auto incoming = [&](int d) { return vm * p.sx[d] * nx + vm * p.sy[d] * ny + vm * p.sz[d] * nz < 0; };
         double a[7] = {0, 0, 0, 0, 0, 0, 0}, acc = 0, a1 = 0, a2 = 0, lat = 0;
-#pragma unroll 4
-        for (int d = 0; d < nd; d++) {
+        // (the refresh alone needs the pass only for a re-emission sum)
+#pragma unroll 8
+        for (int d = 0; d < (MOM || dif || type == 5 ? nd : 0); d++) {
             const double x = row[d * str];
             if constexpr (MOM) {
                 const double *q = wt + kWTab * d;
@@ -2011,24 +2025,36 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
             const double *partner = eb + (size_t)(2 * cb + (s & 1)) * nb + b;
             const double jump = type < 0 ? Cb * (bT - m.b_T[cb]) : 0.0;
             const double *from = (snap && type == 3 ? snap : eb) + (size_t)s * nb + b;
-#pragma unroll 4
-            for (int d = 0; d < nd; d++) {
-                if (!incoming(d)) continue;
-                double val;
-                if (type == 1)
-                    val = Cb * bT;
-                else if (type == 2 || type == 5)
-                    val = acc;
-                else if (type == 3)
-                    val = from[spec_src[(size_t)s * nd + d] * str];
-                else if (type == 6)  // p specular + (1 - p) diffuse, p = the wall's specularity
-                    val = bT * from[spec_src[(size_t)s * nd + d] * str] + (1.0 - bT) * acc;
-                else if (type < 0)
-                    val = partner[d * str] + jump;
-                else
-                    continue;
-                row[d * str] = val;
-                if constexpr (MOM) lat += wt[kWTab * d] * val;
+            const double *src = type < 0 ? partner : from;
+            const bool cst = type == 1 || type == 2 || type == 5, far = type == 3 || type == 6 || type < 0;
+            for (int d0 = 0; (cst || far) && d0 < nd; d0 += kWallBatch) {
+                double x[kWallBatch];
+                unsigned in = 0;
+#pragma unroll
+                for (int i = 0; i < kWallBatch; i++) {
+                    const int d = d0 + i;
+                    if (d >= nd || !incoming(d)) continue;
+                    in |= 1u << i;
+                    if (far) x[i] = src[(type < 0 ? d : spec_src[(size_t)s * nd + d]) * str];
+                }
+#pragma unroll
+                for (int i = 0; i < kWallBatch; i++) {
+                    if (!(in >> i & 1)) continue;
+                    const int d = d0 + i;
+                    double val;
+                    if (type == 1)
+                        val = Cb * bT;
+                    else if (cst)
+                        val = acc;
+                    else if (type == 3)
+                        val = x[i];
+                    else if (type == 6)  // p specular + (1 - p) diffuse, p = the wall's specularity
+                        val = bT * x[i] + (1.0 - bT) * acc;
+                    else
+                        val = x[i] + jump;
+                    row[d * str] = val;
+                    if constexpr (MOM) lat += wt[kWTab * d] * val;
+                }
             }
         }
         if constexpr (MOM) {
@@ -2152,19 +2178,24 @@ __global__ void k_tr_wall_start(DMesh m, DPhys p, const double *__restrict__ e, 
 }
 
 // Margins of a transient step (transient.cpp:818-863), one block in cell
-// order: sum |T - T_old|, max |T|, sum ||q| - |q_old||, max |q|.
-__global__ void k_tr_margins(int nc, const double *__restrict__ T, const double *__restrict__ Told,
-                             const double *__restrict__ q, const double *__restrict__ qold, double *__restrict__ out) {
+// order: sum |T - T_old|, max |T|, sum ||q| - |q_old||, max |q|; and the
+// step's end: T takes the lattice temperature and qold the flux (in place of
+// three copies per step), out[4] the probe's temperature.
+__global__ void k_tr_margins(int nc, int probe, const double *__restrict__ Tlat, double *__restrict__ T,
+                             const double *__restrict__ q, double *__restrict__ qold, double *__restrict__ out) {
     __shared__ double sh[4][1024];
     double a = 0, mt = 0, h = 0, mq = 0;
     for (int i = threadIdx.x; i < nc; i += blockDim.x) {
-        a += fabs(T[i] - Told[i]);
-        mt = fmax(mt, fabs(T[i]));
+        const double Tn = Tlat[i];
+        a += fabs(Tn - T[i]);
+        mt = fmax(mt, fabs(Tn));
+        T[i] = Tn;
         const double q1 = sqrt(q[3 * i] * q[3 * i] + q[3 * i + 1] * q[3 * i + 1] + q[3 * i + 2] * q[3 * i + 2]);
         const double q0 = sqrt(qold[3 * i] * qold[3 * i] + qold[3 * i + 1] * qold[3 * i + 1] +
                                qold[3 * i + 2] * qold[3 * i + 2]);
         h += fabs(q1 - q0);
         mq = fmax(mq, q1);
+        for (int r = 0; r < 3; r++) qold[3 * i + r] = q[3 * i + r];
     }
     sh[0][threadIdx.x] = a, sh[1][threadIdx.x] = mt, sh[2][threadIdx.x] = h, sh[3][threadIdx.x] = mq;
     __syncthreads();
@@ -2178,6 +2209,7 @@ __global__ void k_tr_margins(int nc, const double *__restrict__ T, const double 
         __syncthreads();
     }
     if (threadIdx.x < 4) out[threadIdx.x] = sh[threadIdx.x][0];
+    if (threadIdx.x == 4) out[4] = Tlat[probe];
 }
 
 // cell-only inverse-distance node temperatures
@@ -4296,8 +4328,9 @@ void Solver::launch_walls(bool moments) {
     cudaStream_t s = cfg.stream;
     if (need_snapshot_)
         cudaMemcpyAsync(eb_snap_, eb_, (size_t)nd * mesh.nbs() * nb * 8, cudaMemcpyDeviceToDevice, s);
-    const int cpb = std::max(1, 256 / nb), grid = (n_wall_slots_ + cpb - 1) / cpb;
-    const int thr = (cpb * nb + 31) / 32 * 32;
+    // walls per block: 256 threads' worth, fewer where that leaves SMs without a block
+    const int cpb = std::max(1, std::min(256 / nb, (n_wall_slots_ + 147) / 148));
+    const int grid = (n_wall_slots_ + cpb - 1) / cpb, thr = (cpb * nb + 31) / 32 * 32;
     const double *snap = need_snapshot_ ? eb_snap_ : nullptr;
     if (moments) {
         const size_t smem = ((size_t)nd * kWTab + (size_t)thr * kWallSlots) * sizeof(double);
@@ -4333,7 +4366,6 @@ Error Solver::solve_t(SolveStats &st) {
     // this handle's directions: all of them, or its block of a direction shard
     const int dlo = dlo_, dhi = dhi_ < 0 ? nd : dhi_;
     const bool sharded = xfn_ != nullptr;
-    const int gB = grid_for((size_t)nd * nbs * nb);
     const int gC = (nc + kThreads - 1) / kThreads, gN = (nslot + kThreads - 1) / kThreads;
     // blocks per geometry of the per-geometry reductions
     const int comp_blocks = std::max(1, std::min(148, (nc / ncomp_ + kThreads - 1) / kThreads));
@@ -4478,7 +4510,7 @@ Error Solver::solve_t(SolveStats &st) {
             GL(K_BOUND_OUT, (k_bound_out<S, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_,
                                                                                                    d0, nbt)));
         else if (n_wall_slots_ > 0)
-            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<dir_grid((size_t)n_wall_slots_ * nb, nbt), kThreads, 0, s>>>(
+            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<wall_grid((size_t)n_wall_slots_ * nb, nbt), kThreads, 0, s>>>(
                                 dm_, dp_, eps, (const S *)wall_grad_, n_wall_slots_, wall_side_, Tbase_, gTb_, eb_, d0,
                                 nbt)));
     };
@@ -4666,9 +4698,9 @@ Error Solver::solve_t(SolveStats &st) {
         // of the field and its gradient. The first iteration's gradient
         // would repeat the start's, as nothing between them changes eps: it
         // is left out where the start's face values are still all there
-        // (zeros, or every direction in one batch). A call of five iterations
+        // (zeros, or every direction in one batch). A call of six iterations
         // from a new start on 192,000 tetrahedra x 40 bands x 128 directions
-        // (FP32) takes 250 ms, 283 with the two gradients (18.7 ms each).
+        // (FP32) takes 250 ms, 283 with the two gradients (16 ms each).
         const bool zero = faces && base_is_T_;
         faces_held = zero || (faces && ndb == nd && dlo == 0 && dhi == nd);
         if (zero) {
@@ -5202,7 +5234,7 @@ Error Solver::solve(SolveStats &st) {
 // outgoing and incoming wall pass, the solver's own starting wall values
 // (k_tr_wall_start), then `steps` explicit steps, each: T_old, q_old <- T, q;
 // per direction batch the LSQ gradient of the old e, the explicit update
-// (k_tr_step), the outgoing wall values of the new e with the old gradient
+// (k_tr_step_face in place, or k_tr_step), the outgoing wall values of the new e with the old gradient
 // and the moments; the incoming walls of every direction; the margins.
 // steps = the number of integers below total / dt; a step whose margins are
 // both at or below the limits ends the run, as do 10000 increases in a row.
@@ -5227,15 +5259,30 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
     CUDA_TRY(cudaMemsetAsync(gTb_, 0, (size_t)nc * 24, s));
     k_init_eps<double><<<dir_grid((size_t)nc * nb, nd), kThreads, 0, s>>>(dm_, dp_, T_, Tbase_, eps);
     const double *w = dm_.lsq_w;
-    const int gB = grid_for((size_t)nd * nbs * nb);
     auto gather = [&]() {
         launch_walls(false);
+    };
+    // the steady solver's face-value path where that takes it (face_path)
+    if (face_path()) {
+        Error fe = face_shape<double, DIM>();
+        if (fe.code) return fe;
+    }
+    const bool faces = face_path() && fshape_.tile.B > 0;
+    auto bound_out = [&](int d0, int nbt) {
+        if (!faces)
+            k_bound_out<double, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0, nbt);
+        else if (n_wall_slots_ > 0)
+            k_bound_out_w<double, DIM><<<wall_grid((size_t)n_wall_slots_ * nb, nbt), kThreads, 0, s>>>(
+                dm_, dp_, eps, (const double *)wall_grad_, n_wall_slots_, wall_side_, Tbase_, gTb_, eb_, d0, nbt);
     };
     for (int d0 = 0; d0 < nd; d0 += ndb) {
         const int nbt = std::min(ndb, nd - d0);
         ev.gd0 = d0;
-        k_gradient<double, DIM><<<grid_for((size_t)nbt * nc * nb), kThreads, 0, s>>>(dm_, dp_, w, eps, g, d0, nbt);
-        k_bound_out<double, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0, nbt);
+        if (faces)
+            CUDA_TRY((launch_grad_face<double, DIM>(eps, d0, nbt)));
+        else
+            k_gradient<double, DIM><<<grid_for((size_t)nbt * nc * nb), kThreads, 0, s>>>(dm_, dp_, w, eps, g, d0, nbt);
+        bound_out(d0, nbt);
     }
     gather();
     // the starting wall values: mirror directions searched from direction 0
@@ -5273,7 +5320,6 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
     }
     // the integers n >= 0 below total / dt
     const long long steps = (long long)std::ceil(total / dt);
-    const int gC = (nc + kThreads - 1) / kThreads;
     if (moments_smem() > 48 * 1024) {
         CUDA_TRY((cudaFuncSetAttribute(k_moments<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
         CUDA_TRY((cudaFuncSetAttribute(k_moments<double, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
@@ -5282,29 +5328,35 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
     double errOld = 0, errOldq = 0;
     int errInc = 0;
     st = TransientStats();
+    CUDA_TRY(cudaMemcpyAsync(qold_, q_, (size_t)nc * 24, cudaMemcpyDeviceToDevice, s));
     CUDA_TRY(cudaEventRecord(ev_[0], s));
     for (long long nt = 0; nt < steps; nt++) {
-        CUDA_TRY(cudaMemcpyAsync(Told_, T_, (size_t)nc * 8, cudaMemcpyDeviceToDevice, s));
-        CUDA_TRY(cudaMemcpyAsync(qold_, q_, (size_t)nc * 24, cudaMemcpyDeviceToDevice, s));
         for (int d0 = 0; d0 < nd; d0 += ndb) {
             const int nbt = std::min(ndb, nd - d0);
             const size_t nbe = (size_t)nbt * nc * nb;
             ev.gd0 = d0;
-            k_gradient<double, DIM><<<grid_for(nbe), kThreads, 0, s>>>(dm_, dp_, w, eps, g, d0, nbt);
-            k_tr_step<DIM><<<grid_for(nbe), kThreads, 0, s>>>(dm_, dp_, ev, Told_, eb_, dt, R, d0, nbt);
-            CUDA_TRY(cudaMemcpyAsync(eps + (size_t)d0 * nc * nb, R, nbe * 8, cudaMemcpyDeviceToDevice, s));
-            k_bound_out<double, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0, nbt);
+            if (faces) {
+                CUDA_TRY((launch_grad_face<double, DIM>(eps, d0, nbt)));
+                const int ppd = nb / kPieceBands<double>, cpb = std::max(1, std::min(128, 256 / ppd));
+                const dim3 grid((nc + cpb - 1) / cpb, (nbt + kResDirs - 1) / kResDirs);
+                k_tr_step_face<DIM><<<grid, (cpb * ppd + 31) / 32 * 32, (size_t)kResDirs * cpb * 4 * 8, s>>>(
+                    dm_, dp_, cpb, eps, g, face_mask_, T_, eb_, dt, d0, nbt);
+            } else {
+                k_gradient<double, DIM><<<grid_for(nbe), kThreads, 0, s>>>(dm_, dp_, w, eps, g, d0, nbt);
+                k_tr_step<DIM><<<grid_for(nbe), kThreads, 0, s>>>(dm_, dp_, ev, T_, eb_, dt, R, d0, nbt);
+                CUDA_TRY(cudaMemcpyAsync(eps + (size_t)d0 * nc * nb, R, nbe * 8, cudaMemcpyDeviceToDevice, s));
+            }
+            bound_out(d0, nbt);
             launch_moments(eps, false, d0, nbt, d0 > 0);
         }
         gather();
         // the transient temperature is the lattice one (transient.cpp:789-796)
-        k_copy<<<gC, kThreads, 0, s>>>(Tlat_, T_, nc);
-        k_tr_margins<<<1, 1024, 0, s>>>(nc, T_, Told_, q_, qold_, mg);
-        CUDA_TRY(cudaMemcpyAsync(h_comp_, mg, 4 * 8, cudaMemcpyDeviceToHost, s));
-        if (hist && nt < cap) CUDA_TRY(cudaMemcpyAsync(hist + nt, T_ + probe, 8, cudaMemcpyDeviceToHost, s));
+        k_tr_margins<<<1, 1024, 0, s>>>(nc, probe, Tlat_, T_, q_, qold_, mg);
+        CUDA_TRY(cudaMemcpyAsync(h_pinned_, mg, 5 * 8, cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
         CUDA_TRY(cudaGetLastError());
-        const double err = h_comp_[0] / nc / h_comp_[1], errq = h_comp_[2] / nc / h_comp_[3];
+        const double err = h_pinned_[0] / nc / h_pinned_[1], errq = h_pinned_[2] / nc / h_pinned_[3];
+        if (hist && nt < cap) hist[nt] = h_pinned_[4];
         if (cfg.verbose)
             printf("Iteration #%lld\t Margin per band per cell: Temperature:%.17g Heat Flux:%.17g\n", nt, err, errq);
         if ((err > errOld && errq > errOldq) || std::isnan(err) || std::isnan(errq) || std::isinf(err) ||
