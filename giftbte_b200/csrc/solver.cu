@@ -5941,53 +5941,58 @@ __global__ void k_adj_ebin(DMesh m, DPhys p, const double *__restrict__ tvc, con
     }
 }
 
-// k_adj_gradT for BC consecutive bands per thread
-template <int DIM, int BC>
-__global__ void __launch_bounds__(256) k_adj_gradT4(DMesh m, DPhys p, const double *__restrict__ tvc,
+// k_adj_gradT for a pair of bands and ND directions per thread (nb even): the
+// stencil's indices and weights are read once for all of them and 2 ND or 3 ND
+// independent 16-byte gathers are in flight per entry. Bound by the latency of
+// those gathers; a thread per four bands of one direction had four behind
+// every index: 101 -> 82 us on 6,488 triangles x 20 bands x 32
+// directions.
+constexpr int kAdjDirs = 4;
+template <int DIM, int ND>
+__global__ void __launch_bounds__(256) k_adj_gradT2(DMesh m, DPhys p, const double *__restrict__ tvc,
                                                     const int *__restrict__ tptr, const int *__restrict__ tidx,
                                                     const double *__restrict__ tw, const double *__restrict__ wsum,
                                                     const int *__restrict__ opp, const int *__restrict__ pos_of,
                                                     const double *__restrict__ ebar, const double *__restrict__ gbar,
                                                     double *__restrict__ Rlo) {
-    const int nb = p.nb, nc = m.nc, nbc = nb / BC;
-    const size_t total = (size_t)p.nd * nc * nbc;
-    for (size_t t = gtid(); t < total; t += gstride()) {
-        const int b0 = BC * (int)(t % nbc);
-        const size_t dc = t / nbc;
-        const int j = (int)(dc % nc);
-        const int d = (int)(dc / nc);
-        const double *gd = gbar + ((size_t)d * nc) * DIM * nb + b0;
-        double acc[BC], gx[BC], gy[BC], gz[BC];
-        ld8(ebar + dc * nb + b0, acc);
-        for (int q = tptr[j]; q < tptr[j + 1]; q++) {
-            const double *g = gd + (size_t)tidx[q] * DIM * nb;
-            const double wx = tw[3 * q], wy = tw[3 * q + 1], wz = tw[3 * q + 2];
-            ld8(g, gx);
-            ld8(g + nb, gy);
-            if (DIM == 3) ld8(g + 2 * nb, gz);
+    const int nb = p.nb, nc = m.nc, nbc = nb / 2;
+    const size_t t = gtid();
+    if (t >= (size_t)nc * nbc) return;
+    const int j = (int)(t / nbc), b0 = 2 * (int)(t % nbc), d0 = blockIdx.y * ND, last = p.nd - 1;
+    double acc[ND][2];
+    const double *gd[ND];
 #pragma unroll
-            for (int i = 0; i < BC; i++) {
-                acc[i] += wx * gx[i] + wy * gy[i];
-                if (DIM == 3) acc[i] += wz * gz[i];
-            }
+    for (int i = 0; i < ND; i++) {
+        const size_t d = min(d0 + i, last);
+        ld8(ebar + (d * nc + j) * nb + b0, acc[i]);
+        gd[i] = gbar + d * nc * DIM * nb + b0;
+    }
+    auto add = [&](size_t at, double wx, double wy, double wz) {
+        double gx[ND][2], gy[ND][2], gz[ND][2];
+#pragma unroll
+        for (int i = 0; i < ND; i++) {
+            ld8(gd[i] + at, gx[i]);
+            ld8(gd[i] + at + nb, gy[i]);
+            if (DIM == 3) ld8(gd[i] + at + 2 * nb, gz[i]);
         }
-        {
-            const double *g = gd + (size_t)j * DIM * nb;
-            const double wx = wsum[3 * j], wy = wsum[3 * j + 1], wz = wsum[3 * j + 2];
-            ld8(g, gx);
-            ld8(g + nb, gy);
-            if (DIM == 3) ld8(g + 2 * nb, gz);
 #pragma unroll
-            for (int i = 0; i < BC; i++) {
-                acc[i] -= wx * gx[i] + wy * gy[i];
-                if (DIM == 3) acc[i] -= wz * gz[i];
+        for (int i = 0; i < ND; i++)
+#pragma unroll
+            for (int v = 0; v < 2; v++) {
+                acc[i][v] += wx * gx[i][v] + wy * gy[i][v];
+                if (DIM == 3) acc[i][v] += wz * gz[i][v];
             }
-        }
-        const double tv = tvc[j];
+    };
+    for (int q = tptr[j]; q < tptr[j + 1]; q++)
+        add((size_t)tidx[q] * DIM * nb, tw[3 * q], tw[3 * q + 1], tw[3 * q + 2]);
+    add((size_t)j * DIM * nb, -wsum[3 * j], -wsum[3 * j + 1], -wsum[3 * j + 2]);
+    const double tv = tvc[j];
 #pragma unroll
-        for (int i = 0; i < BC; i++) acc[i] *= tv;
-        const int od = opp[d];
-        st8(Rlo + ((size_t)od * nc + pos_of[(size_t)od * nc + j]) * nb + b0, acc);
+    for (int i = 0; i < ND; i++) {
+        if (d0 + i > last) continue;
+        const int od = opp[d0 + i];
+        acc[i][0] *= tv, acc[i][1] *= tv;
+        st8(Rlo + ((size_t)od * nc + pos_of[(size_t)od * nc + j]) * nb + b0, acc[i]);
     }
 }
 
@@ -6149,14 +6154,19 @@ __global__ void __launch_bounds__(256) k_aa_dots(size_t n, int mh, AAVecs H, con
     for (int i = 0; i < 2 * (kAAMax + 1); i++) acc[i] = 0;
     for (size_t t = gtid(); t < n; t += gstride()) {
         const double fv = f[t], d = fv - fprev[t];
+        // (the stored vectors are read before the stores, which the compiler
+        // cannot move loads across: 73 -> 57 us for 4.1
+        // million values and six stored vectors)
+        double h[kAAMax];
+#pragma unroll
+        for (int i = 0; i < kAAMax; i++) h[i] = i < mh ? H.df[i][t] : 0.0;
         dfn[t] = d;
         fprev[t] = fv;
 #pragma unroll
         for (int i = 0; i < kAAMax; i++)
             if (i < mh) {
-                const double h = H.df[i][t];
-                acc[2 * i] += d * h;
-                acc[2 * i + 1] += fv * h;
+                acc[2 * i] += d * h[i];
+                acc[2 * i + 1] += fv * h[i];
             }
         acc[2 * kAAMax] += d * d;
         acc[2 * kAAMax + 1] += fv * d;
@@ -6195,12 +6205,22 @@ __global__ void k_aa_update(size_t n, int mh, AAHist H, const double *__restrict
     }
 }
 
-// sum of squares of x[0 .. n) into *out (atomics per warp)
-__global__ void k_sqnorm(size_t n, const double *__restrict__ x, double *out) {
+// sum of squares of x[0 .. n) into *out: four blocks per SM, one atomic per
+// block (an atomic per warp of a thread per value was 117 us for 4.1 million
+// values, all of it the queue at the one address; now 9.8)
+constexpr int kSqBlocks = 4 * 148;
+__global__ void __launch_bounds__(kThreads) k_sqnorm(size_t n, const double *__restrict__ x, double *out) {
+    __shared__ double sh[kThreads / 32];
     double s2 = 0;
+#pragma unroll 4
     for (size_t t = gtid(); t < n; t += gstride()) s2 += x[t] * x[t];
     s2 = warp_sum(s2);
-    if ((threadIdx.x & 31) == 0) atomicAdd(out, s2);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s2;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < kThreads / 32; i++) s2 += sh[i];
+        atomicAdd(out, s2);
+    }
 }
 
 __global__ void k_adj_update(DMesh m, DPhys p, const int *__restrict__ opp, const double *__restrict__ Dc,
@@ -6267,74 +6287,117 @@ __global__ void k_adj_u(DMesh m, const double *__restrict__ Q, const double *__r
     U[c] = acc + m.heat[c] * m.vol[c];
 }
 
-// gradient assembly over cells: warp per cell, lanes over (direction, band).
+// Gradient assembly over cells, a thread per (cell, band) walking the
+// directions (blockDim = cpb * nb, rounded up to a warp).
 // Gamma = lam (e - C_b T*) gives the residual's tau and s_c derivatives; the
-// tensor moment's tau derivative is v_b^2 (w s s^T e) : Qbar. Per-band sums
-// go through shared memory (nb <= 256) into g_tau.
-__global__ void k_adj_assemble(DMesh m, DPhys p, const double *__restrict__ lam, const double *__restrict__ eps,
-                               const double *__restrict__ T, const double *__restrict__ Qbar, double *g_cell,
-                               double *g_tau) {
-    extern __shared__ double sb[];
-    for (int i = threadIdx.x; i < p.nb; i += blockDim.x) sb[i] = 0;
-    __syncthreads();
-    const int c = (int)(gtid() >> 5), lane = threadIdx.x & 31;
-    if (c < m.nc) {
-        const int n = p.nd * p.nb;
+// tensor moment's tau derivative is v_b^2 (w s s^T e) : Qbar. Sums over the
+// block's cells per band and over a cell's bands go through shared memory,
+// one atomic per band and block into g_tau. Bound by reading lam and e; a
+// warp per cell with lanes over (direction, band) and a shared-memory FP64
+// atomic per value: 54 -> 27 us on 6,488 triangles x 20 bands x 32
+// directions.
+__global__ void __launch_bounds__(256) k_adj_assemble(DMesh m, DPhys p, int cpb, const double *__restrict__ lam,
+                                                      const double *__restrict__ eps, const double *__restrict__ T,
+                                                      const double *__restrict__ Qbar, double *g_cell, double *g_tau) {
+    __shared__ double sg[256], st[256];
+    const int nb = p.nb, ci = threadIdx.x / nb, b = threadIdx.x % nb, c = blockIdx.x * cpb + ci;
+    double gs = 0, ts = 0;
+    if (ci < cpb && c < m.nc) {
+        const double ct = p.C[b] * T[c], f = p.tau[b] * p.vmag[b] * p.vmag[b];
         const double *q = Qbar + 6 * (size_t)c;
-        double gs = 0;
-        for (int i = lane; i < n; i += 32) {
-            const int d = i / p.nb, b = i % p.nb;
-            const double e = eps[((size_t)d * m.nc + c) * p.nb + b];
-            const double G = lam[((size_t)d * m.nc + c) * p.nb + b] * (e - p.C[b] * T[c]);
+        const double q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];
+        const bool syn = p.hr[b] > 0;
+        const size_t row = (size_t)m.nc * nb;
+        const double *ep = eps + (size_t)c * nb + b, *lp = lam + (size_t)c * nb + b;
+#pragma unroll 8
+        for (int d = 0; d < p.nd; d++) {
+            const double e = ep[d * row];
+            const double G = lp[d * row] * (e - ct);
             gs += G;
             double tb = G;  // d/d(ln tau_b) of the residual
-            if (p.hr[b] > 0) {
+            if (syn) {
                 const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
-                tb += p.tau[b] * p.vmag[b] * p.vmag[b] * p.w[d] * e *
-                      (q[0] * sx * sx + q[1] * sx * sy + q[2] * sx * sz + q[3] * sy * sy + q[4] * sy * sz + q[5] * sz * sz);
+                tb += f * p.w[d] * e * (q0 * sx * sx + q1 * sx * sy + q2 * sx * sz + q3 * sy * sy + q4 * sy * sz + q5 * sz * sz);
             }
-            atomicAdd(&sb[b], tb);
+            ts += tb;
         }
-        gs = warp_sum(gs);
-        if (lane == 0) g_cell[c] = -gs * m.tsc[c];
     }
+    sg[threadIdx.x] = gs;
+    st[threadIdx.x] = ts;
     __syncthreads();
-    for (int i = threadIdx.x; i < p.nb; i += blockDim.x) atomicAdd(&g_tau[i], sb[i]);
+    const int ncell = min(cpb, m.nc - (int)blockIdx.x * cpb);
+    for (int i = threadIdx.x; i < nb + ncell; i += blockDim.x) {
+        double sum = 0;
+        if (i < nb) {
+            for (int k = 0; k < ncell; k++) sum += st[k * nb + i];
+            atomicAdd(&g_tau[i], sum);
+        } else {
+            const int k = i - nb, cc = blockIdx.x * cpb + k;
+            for (int bb = 0; bb < nb; bb++) sum += sg[k * nb + bb];
+            g_cell[cc] = -sum * m.tsc[cc];
+        }
+    }
 }
 
 // the tensor moment's tau derivative on wall sides, and the specularity
-// derivative of partially specular walls: warp per side
-__global__ void k_adj_assemble_sides(DMesh m, DPhys p, const double *__restrict__ eb, const double *__restrict__ ebb,
-                                     const double *__restrict__ dsum, const int *__restrict__ spec_src,
-                                     const double *__restrict__ Qsbar, double *g_tau, double *g_bnd) {
-    extern __shared__ double sb[];
-    for (int i = threadIdx.x; i < p.nb; i += blockDim.x) sb[i] = 0;
-    __syncthreads();
-    const int s = (int)(gtid() >> 5), lane = threadIdx.x & 31;
-    if (s < m.nbs && m.bs_cell[s] >= 0) {
-        const int n = p.nd * p.nb, k = m.bs_cf[s], ib = s >> 1;
+// derivative of partially specular walls: a thread per (side, band) walking
+// the directions, sums as in k_adj_assemble (a warp per side with atomics per
+// value: 28.6 -> 27.3 us for 732 wall sides x 20 bands x 32 directions)
+__global__ void __launch_bounds__(256) k_adj_assemble_sides(DMesh m, DPhys p, int cpb, const double *__restrict__ eb,
+                                                            const double *__restrict__ ebb,
+                                                            const double *__restrict__ dsum,
+                                                            const int *__restrict__ spec_src,
+                                                            const double *__restrict__ Qsbar, double *g_tau,
+                                                            double *g_bnd) {
+    __shared__ double sp[256], st[256];
+    const int nb = p.nb, li = threadIdx.x / nb, b = threadIdx.x % nb, s = blockIdx.x * cpb + li;
+    double gp = 0, ts = 0;
+    if (li < cpb && s < m.nbs && m.bs_cell[s] >= 0 && p.hr[b] > 0) {
+        const int k = m.bs_cf[s];
+        const bool partial = m.b_type[s >> 1] == 6;
+        const double f = p.tau[b] * p.vmag[b] * p.vmag[b];
+        const double nx = m.cf_nx[k], ny = m.cf_ny[k], nz = m.cf_nz[k];
         const double *q = Qsbar + 6 * (size_t)s;
-        const bool partial = m.b_type[ib] == 6;
-        double gp = 0;
-        for (int i = lane; i < n; i += 32) {
-            const int d = i / p.nb, b = i % p.nb;
-            if (!(p.hr[b] > 0)) continue;
+        const double q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];
+        const size_t row = (size_t)m.nbs * nb, at = (size_t)s * nb + b;
+#pragma unroll 8
+        for (int d = 0; d < p.nd; d++) {
             const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
-            const double x = eb[((size_t)d * m.nbs + s) * p.nb + b];
-            atomicAdd(&sb[b], p.tau[b] * p.vmag[b] * p.vmag[b] * p.w[d] * x *
-                                  (q[0] * sx * sx + q[1] * sx * sy + q[2] * sx * sz + q[3] * sy * sy + q[4] * sy * sz +
-                                   q[5] * sz * sz));
-            if (partial && sx * m.cf_nx[k] + sy * m.cf_ny[k] + sz * m.cf_nz[k] < 0) {
-                const int src = spec_src[(size_t)s * p.nd + d];
-                gp += ebb[((size_t)d * m.nbs + s) * p.nb + b] *
-                      (eb[((size_t)src * m.nbs + s) * p.nb + b] - dsum[(size_t)s * p.nb + b]);
-            }
+            const double x = eb[d * row + at];
+            ts += f * p.w[d] * x * (q0 * sx * sx + q1 * sx * sy + q2 * sx * sz + q3 * sy * sy + q4 * sy * sz + q5 * sz * sz);
         }
-        gp = warp_sum(gp);
-        if (lane == 0 && partial) atomicAdd(&g_bnd[ib], gp);
+        // (every load of a batch before its first use)
+        const double dif = partial ? dsum[at] : 0.0;
+        for (int d0 = 0; partial && d0 < p.nd; d0 += 8) {
+            double y[8], z[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const int d = min(d0 + i, p.nd - 1);
+                const bool in = d0 + i < p.nd && p.sx[d] * nx + p.sy[d] * ny + p.sz[d] * nz < 0;
+                y[i] = eb[(in ? spec_src[(size_t)s * p.nd + d] : d) * row + at];
+                z[i] = in ? ebb[d * row + at] : 0.0;
+                if (!in) y[i] = dif;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++) gp += z[i] * (y[i] - dif);
+        }
     }
+    sp[threadIdx.x] = gp;
+    st[threadIdx.x] = ts;
     __syncthreads();
-    for (int i = threadIdx.x; i < p.nb; i += blockDim.x) atomicAdd(&g_tau[i], sb[i]);
+    const int ns = min(cpb, m.nbs - (int)blockIdx.x * cpb);
+    for (int i = threadIdx.x; i < nb + ns; i += blockDim.x) {
+        double sum = 0;
+        if (i < nb) {
+            for (int k = 0; k < ns; k++) sum += st[k * nb + i];
+            atomicAdd(&g_tau[i], sum);
+        } else {
+            const int k = i - nb, ss = blockIdx.x * cpb + k;
+            if (m.bs_cell[ss] < 0 || m.b_type[ss >> 1] != 6) continue;
+            for (int bb = 0; bb < nb; bb++) sum += sp[k * nb + bb];
+            atomicAdd(&g_bnd[ss >> 1], sum);
+        }
+    }
 }
 
 }  // namespace
@@ -6493,7 +6556,6 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
     const int gC = (nc + kThreads - 1) / kThreads, gN = (nslot + kThreads - 1) / kThreads;
     const int gS = (nbs + kThreads - 1) / kThreads;
     const int gWc = (int)(((size_t)nc * 32 + kThreads - 1) / kThreads);
-    const int gWs = (int)(((size_t)nbs * 32 + kThreads - 1) / kThreads);
     const double kappa = dp_.kappa;
     // sweep launch (FP64 records; the forward's band chunking)
     constexpr int LOOK = 4, LCAP = 128;
@@ -6590,13 +6652,14 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
     // the rest of A^-T [(dF/de)^T L + dJ/de] after evaluate(): the
     // gradient's transpose, the opposite-direction sweep
     auto finish = [&]() -> Error {
-        if (nb % 4 == 0) {
+        if (nb % 2 == 0) {
+            const dim3 grid((unsigned)(((size_t)nc * (nb / 2) + kThreads - 1) / kThreads), (nd + kAdjDirs - 1) / kAdjDirs);
             if (dim == 2)
-                k_adj_gradT4<2, 4><<<grid_for(ne / 4), kThreads, 0, s>>>(dm_, dp_, tvc, tptr, tidx, tw, wsum, opp,
-                                                                         pos_of_, ebar, gbar, Rlo);
+                k_adj_gradT2<2, kAdjDirs><<<grid, kThreads, 0, s>>>(dm_, dp_, tvc, tptr, tidx, tw, wsum, opp, pos_of_,
+                                                                    ebar, gbar, Rlo);
             else
-                k_adj_gradT4<3, 4><<<grid_for(ne / 4), kThreads, 0, s>>>(dm_, dp_, tvc, tptr, tidx, tw, wsum, opp,
-                                                                         pos_of_, ebar, gbar, Rlo);
+                k_adj_gradT2<3, kAdjDirs><<<grid, kThreads, 0, s>>>(dm_, dp_, tvc, tptr, tidx, tw, wsum, opp, pos_of_,
+                                                                    ebar, gbar, Rlo);
         } else if (dim == 2) {
             k_adj_gradT<2><<<grid_for(ne), kThreads, 0, s>>>(dm_, dp_, tptr, tidx, tw, wsum, opp, pos_of_, ebar, gbar,
                                                               Rlo);
@@ -6619,8 +6682,10 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
     const double mdim = bands.material_dim == 2 ? 2.0 : 3.0;
     auto assemble = [&](std::vector<double> &gt, std::vector<double> &gc, std::vector<double> &gb) -> Error {
         CUDA_TRY(cudaMemsetAsync(gtau, 0, (size_t)(nb + nbd) * 8, s));
-        k_adj_assemble<<<gWc, kThreads, nb * 8, s>>>(dm_, dp_, lam, eps, T_, Qbar, gcell, gtau);
-        k_adj_assemble_sides<<<gWs, kThreads, nb * 8, s>>>(dm_, dp_, eb_, ebb, dsum_, spec_src_, Qsbar, gtau, gbnd);
+        const int cpb = std::max(1, kThreads / nb), thr = (cpb * nb + 31) / 32 * 32;
+        k_adj_assemble<<<(nc + cpb - 1) / cpb, thr, 0, s>>>(dm_, dp_, cpb, lam, eps, T_, Qbar, gcell, gtau);
+        k_adj_assemble_sides<<<(nbs + cpb - 1) / cpb, thr, 0, s>>>(dm_, dp_, cpb, eb_, ebb, dsum_, spec_src_, Qsbar,
+                                                                   gtau, gbnd);
         CUDA_TRY(cudaGetLastError());
         gt.resize(nb);
         gc.resize(nc);
@@ -6683,7 +6748,7 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
         ee = finish();  // Rlo = r(lam) in level order, then A^-T r(lam)
         if (ee.code) return ee;
         CUDA_TRY(cudaMemsetAsync(red, 0, 8, s));
-        k_sqnorm<<<grid_for(ne), kThreads, 0, s>>>(ne, Rlo, red);
+        k_sqnorm<<<std::min(grid_for(ne), kSqBlocks), kThreads, 0, s>>>(ne, Rlo, red);
         CUDA_TRY(cudaGetLastError());
         double r2 = 0;
         CUDA_TRY(cudaMemcpyAsync(&h_pinned_[10], red, 8, cudaMemcpyDeviceToHost, s));
