@@ -5,13 +5,17 @@
 // (band, direction) pairs at once (they are independent within an iteration:
 // temperatureOld is frozen by copy() and incoming boundary values are only
 // refreshed after the pair loop):
-//   k_gradient   LSQ gradient over the vertex-neighbour stencil
-//                (_get_gradient_larger, StaticBTESynthetic.cpp:1243-1424)
-//   k_residual   second-order upwind defect R(e) (_get_Re, :1427-1500)
+//   k_grad_face  LSQ gradient over the vertex-neighbour stencil
+//                (_get_gradient_larger, StaticBTESynthetic.cpp:1243-1424) and
+//                the upwind face values it gives (k_gradient*: gradient
+//                arrays, where Solver::face_path does not apply)
+//   k_resid_face second-order upwind defect R(e) (_get_Re, :1427-1500)
+//                (k_residual*: from gradient arrays)
 //   k_sweep      d = A^-1 R with A the first-order upwind operator
 //                (_get_coefficient :784-840), by a level-scheduled wavefront
 //                sweep per direction instead of a sparse LU; e += d
-//   k_bound_out  outgoing boundary values (_get_bound_ee, :1502-1539)
+//   k_bound_out_w, k_bound_out  outgoing boundary values (_get_bound_ee,
+//                :1502-1539)
 //   k_moments    T, T_band, E, q (:2487-2520) plus the two moments the
 //                synthetic source needs
 //   k_remacro    the non-Fourier source (_set_vertex_energydensity,
@@ -20,10 +24,11 @@
 //                band/direction weights that factor out of the face and
 //                vertex stencils, so the per-pair face pass collapses into
 //                one pass over cells per iteration
-//   k_gather     incoming boundary values by wall type (_set_bound_ee_1,
-//                :2083-2232)
-//   macro        boundary temperatures (:2234-2274), Picard loop of FP64
-//                Jacobi-preconditioned CG solves of the Fourier system
+//   k_walls      incoming boundary values by wall type (_set_bound_ee_1,
+//                :2083-2232), the walls' moments and their macro
+//                temperatures (:2234-2274)
+//   macro        Picard loop of FP64 preconditioned CG solves of the Fourier
+//                system
 //                (_marco_solution :2692-2734, _get_Re_macro :2307-2407)
 //   margins      (_get_magin_check_error, :2565-2611)
 // Band intensities are stored as a deviation from C_b * T_base[c]; the FP64
@@ -2725,8 +2730,8 @@ __global__ void __launch_bounds__(kCgThreads, 1)
                  const int *__restrict__ perm, const double *__restrict__ ell_val, const int *__restrict__ ell_col,
                  const double *__restrict__ diag, const int *__restrict__ agg_ptr, const double *__restrict__ ainv,
                  const int *__restrict__ nsend, const int *__restrict__ snd_src, const int *__restrict__ snd_dst,
-                 const double *__restrict__ bvec, double *__restrict__ x, double rtol, double eta, int maxit,
-                 const double *__restrict__ t1, double *__restrict__ out) {
+                 const double *__restrict__ bvec, const double *x0, double *x, double *keep, double rtol, double eta,
+                 int maxit, const double *t1, double *__restrict__ out) {
     cgrp::cluster_group cl = cgrp::this_cluster();
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int NA = C * kCgAgg;  // aggregates in all (<= kCgThreads)
@@ -2750,7 +2755,7 @@ __global__ void __launch_bounds__(kCgThreads, 1)
     const int base = part_ptr[rank], nr = part_ptr[rank + 1] - base, ns = nsend[rank];
     for (int i = tid; i < nr; i += bd) {
         const int o = perm[base + i];
-        xs[i] = x[o];
+        xs[i] = x0[o];
         us[i] = xs[i];
         rs[i] = bvec[o];
         dg[i] = diag[base + i];
@@ -2998,11 +3003,12 @@ __global__ void __launch_bounds__(kCgThreads, 1)
     double sq = 0;
     for (int i = tid; i < nr; i += bd) {
         const int o = perm[base + i];
-        x[o] = xs[i];
         if (t1) {
-            const double dd = xs[i] - t1[o];
+            const double dd = xs[i] - t1[o];  // (t1 may be x: its values before this solve)
             sq += dd * dd;
         }
+        x[o] = xs[i];
+        if (keep) keep[o] = xs[i];
     }
     if (t1) {
         sq = warp_allsum(sq);
@@ -4135,14 +4141,16 @@ Error Solver::cg_plan(const std::vector<int> &ptr, const std::vector<int> &idx, 
     return {0, ""};
 }
 
-// Jacobi-preconditioned CG on a negated (SPD) CSR system, from the initial
-// guess in x. With a cluster plan the whole solve runs in one
-// cluster-resident kernel;
-// otherwise in the grid-wide cooperative kernel, with scratch vectors and
-// 65536 reduction slots passed in by the caller. When t1 is given, *sq
-// receives sum (x - t1)^2 of the solution. Waits for the stream.
+// Preconditioned CG on a negated (SPD) CSR system, from the initial guess in
+// x, or in warm with use_warm. With a cluster plan the whole solve runs in one
+// cluster-resident kernel; otherwise in the grid-wide cooperative kernel, with
+// scratch vectors and exchange slots passed in by the caller. When t1 is given,
+// *sq receives sum (x - t1)^2 of the solution; with a cluster plan t1 may be x
+// (its values before the solve). warm, when given, receives the solution too:
+// the cluster kernel reads and writes both itself, in place of two copies
+// around a launch of 40 to 200 us. Waits for the stream.
 Error Solver::cg_solve(const CgPlan &pl, const double *dinv, double *x, const double *b, double rtol, double eta, long long &iters, double *scal, double *r,
-                       double *z, double *p, double *Ap, const double *t1, double *sq) {
+                       double *z, double *p, double *Ap, const double *t1, double *sq, double *warm, bool use_warm) {
     cudaStream_t s = cfg.stream;
     int n = mesh.nc;
     int maxit = 20000;
@@ -4164,7 +4172,8 @@ Error Solver::cg_solve(const CgPlan &pl, const double *dinv, double *x, const do
                                             (const int *)pl.part_ptr, (const int *)pl.perm, (const double *)pl.ell_val,
                                             (const int *)pl.ell_col, (const double *)pl.diag, (const int *)pl.agg_ptr,
                                             (const double *)pl.ainv, (const int *)pl.nsend, (const int *)pl.snd_src,
-                                            (const int *)pl.snd_dst, b, x, rtol, eta, maxit, t1, scal));
+                                            (const int *)pl.snd_dst, b, use_warm ? (const double *)warm : x, x, warm, rtol, eta,
+                                            maxit, t1, scal));
         CUDA_TRY(lerr);
         CUDA_TRY(cudaMemcpyAsync(h_pinned_ + 8, scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
@@ -4173,6 +4182,7 @@ Error Solver::cg_solve(const CgPlan &pl, const double *dinv, double *x, const do
         if (sq) *sq = t1 ? h_pinned_[9] : 0.0;
         return {0, ""};
     }
+    if (use_warm) CUDA_TRY(cudaMemcpyAsync(x, warm, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
     // rows per thread in registers (up to 4), or none where the grid's
     // threads hold fewer than the system's rows that way
     int R = 1;
@@ -4199,6 +4209,7 @@ Error Solver::cg_solve(const CgPlan &pl, const double *dinv, double *x, const do
     if (h_pinned_[9] < 0) return {-5, "the grid-wide CG lost an exchange between its blocks"};
     iters += (long long)h_pinned_[9];
     if (sq) *sq = t1 ? h_pinned_[8] : 0.0;
+    if (warm) CUDA_TRY(cudaMemcpyAsync(warm, x, (size_t)n * 8, cudaMemcpyDeviceToDevice, s));
     return {0, ""};
 }
 
@@ -5094,7 +5105,10 @@ Error Solver::solve_t(SolveStats &st) {
         std::vector<char> done(ncomp_, 0);
         if (ncomp_ > 1) CUDA_TRY(cudaMemsetAsync(comp_done_d_, 0, sizeof(int) * ncomp_, s));
         while (internal > 1e-6) {
-            GL(K_COPY, k_copy<<<gC, kThreads, 0, s>>>(T_, T1_, nc));
+            // the iterate before this step: the cluster CG compares with T_
+            // itself, the grid-wide one and a batch's tests need the copy
+            const bool before = !kplan_.C || ncomp_ > 1;
+            if (before) GL(K_COPY, k_copy<<<gC, kThreads, 0, s>>>(T_, T1_, nc));
             GL(K_TINTERP, k_tinterp<<<gN, kThreads, 0, s>>>(dm_, T_, TV_));
             GL(K_MACRO_RHS, k_macro_rhs<<<gC, kThreads, 0, s>>>(dm_, dp_.kappa, dp_.kap, dp_.mat, remacro_, bTm_, TV_,
                                                                rhs_));
@@ -5102,26 +5116,21 @@ Error Solver::solve_t(SolveStats &st) {
             // warm start from this Picard step's solution of the previous
             // outer iteration; tolerance tightens with the outer margin
             const int step = inner;
-            if (step < (int)warm_.size() && warm_[step] && warm_ok_[step])
-                CUDA_TRY(cudaMemcpyAsync(T_, warm_[step], (size_t)nc * 8, cudaMemcpyDeviceToDevice, s));
+            if (step >= (int)warm_.size()) {
+                warm_.resize(step + 1, nullptr);
+                warm_ok_.resize(step + 1, 0);
+            }
+            if (!warm_[step]) warm_[step] = (double *)dalloc((size_t)nc * 8);
+            const bool held = warm_[step] && warm_ok_[step];
             // from a warm start the residual must drop by kWarmEta; the
             // absolute floor macro_rtol * |b| still bounds the final error
-            const bool warm = step < (int)warm_.size() && warm_[step] && warm_ok_[step] && !cfg.macro_exact;
+            const bool warm = held && !cfg.macro_exact;
             double sq = 0;
-            Error e = cg_solve(kplan_, K_dinv_, T_, rhs_, cfg.macro_rtol,
-                               warm ? kWarmEta : 0.0, st.cg_iterations, cg_scal_, cg_r_, cg_z_, cg_p_, cg_Ap_, T1_, &sq);
+            warm_ok_[step] = 0;
+            Error e = cg_solve(kplan_, K_dinv_, T_, rhs_, cfg.macro_rtol, warm ? kWarmEta : 0.0, st.cg_iterations,
+                               cg_scal_, cg_r_, cg_z_, cg_p_, cg_Ap_, before ? T1_ : T_, &sq, warm_[step], held);
             prof_collect(st);
-            if (!e.code) {
-                if (step >= (int)warm_.size()) {
-                    warm_.resize(step + 1, nullptr);
-                    warm_ok_.resize(step + 1, 0);
-                }
-                if (!warm_[step]) warm_[step] = (double *)dalloc((size_t)nc * 8);
-                if (warm_[step]) {
-                    CUDA_TRY(cudaMemcpyAsync(warm_[step], T_, (size_t)nc * 8, cudaMemcpyDeviceToDevice, s));
-                    warm_ok_[step] = 1;
-                }
-            }
+            if (!e.code && warm_[step]) warm_ok_[step] = 1;
             if (e.code) return e;
             internal = sq / nc;
             if (ncomp_ > 1) {
@@ -5616,7 +5625,7 @@ __global__ void k_adj_neg(const double *__restrict__ x, double *__restrict__ y, 
 }
 
 // transpose of the side-moment and wall-temperature reads of one wall entry
-// (k_side_moments, k_macro_bc): the cotangent of eb[d][s][b]
+// (k_walls): the cotangent of eb[d][s][b]
 __device__ __forceinline__ double adj_side_entry(const DMesh &m, const DPhys &p, int d, int s, int b,
                                                  const double *Thsbar, const double *Qsbar, const double *bTmbar) {
     const double w = p.w[d], Cb = p.C[b];
@@ -6018,7 +6027,7 @@ __global__ void k_adj_dsum(DMesh m, DPhys p, const double *__restrict__ ebb, dou
 }
 
 // outgoing wall entries: side-moment cotangent plus the transpose of the
-// incoming gather (k_diffuse_sum + k_gather) from this side or, for
+// incoming values (k_walls) from this side or, for
 // periodic walls, from the sides that read it
 __global__ void k_adj_ebout(DMesh m, DPhys p, const double *__restrict__ dif_w, const int *__restrict__ sinv_ptr,
                             const int *__restrict__ sinv_idx, const double *__restrict__ dbar, const int *__restrict__ per_ptr,
@@ -6596,14 +6605,10 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
         CUDA_TRY(cudaMemsetAsync(zsum, 0, (size_t)nc * 8, s));
         for (int k = N - 1; k >= 0; k--) {
             double *wk = adj_warm_ + (size_t)k * nc;
-            if (warm)
-                CUDA_TRY(cudaMemcpyAsync(z, wk, (size_t)nc * 8, cudaMemcpyDeviceToDevice, s));
-            else
-                CUDA_TRY(cudaMemsetAsync(z, 0, (size_t)nc * 8, s));
-            Error ce = cg_solve(kplan_, K_dinv_, z, Tb, cfg.macro_rtol, warm ? kWarmEta : 0.0,
-                                cg_its, cg_scal_, cg_r_, cg_z_, cg_p_, cg_Ap_, nullptr, nullptr);
+            if (!warm) CUDA_TRY(cudaMemsetAsync(z, 0, (size_t)nc * 8, s));
+            Error ce = cg_solve(kplan_, K_dinv_, z, Tb, cfg.macro_rtol, warm ? kWarmEta : 0.0, cg_its, cg_scal_, cg_r_,
+                                cg_z_, cg_p_, cg_Ap_, nullptr, nullptr, wk, warm);
             if (ce.code) return ce;
-            CUDA_TRY(cudaMemcpyAsync(wk, z, (size_t)nc * 8, cudaMemcpyDeviceToDevice, s));
             CUDA_TRY(cudaMemsetAsync(TVbar, 0, (size_t)nslot * 8, s));
             k_adj_macro_tv<<<gC, kThreads, 0, s>>>(dm_, kappa, z, TVbar);
             CUDA_TRY(cudaMemsetAsync(Tb, 0, (size_t)nc * 8, s));

@@ -228,7 +228,7 @@ private:
     Error alloc_all();
     Error cg_solve(const CgPlan &pl, const double *dinv, double *x, const double *b, double rtol, double eta,
                    long long &iters, double *scal, double *r, double *z, double *p, double *Ap, const double *t1,
-                   double *sq);
+                   double *sq, double *warm = nullptr, bool use_warm = false);
     Error ell_plan(const std::vector<int> &ptr, const std::vector<int> &idx, const std::vector<double> &val,
                    CgPlan &pl);
     Error cg_plan(const std::vector<int> &ptr, const std::vector<int> &idx, const std::vector<double> &val,
