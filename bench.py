@@ -128,18 +128,21 @@ class ClockSampler:
 
 # Algorithmic bytes of one launch of each kernel: the least DRAM traffic its
 # work needs. s = bytes of a stored intensity (4 in the FP32 form, 8 in
-# FP64), dim = stored gradient components, rec = bytes of one sweep record
-# (per direction and cell). Per band*direction*cell update unless noted:
-#   gradient  read e, write g                         (1 + dim) s
-#   residual  read e and g, write R                   (2 + dim) s
+# FP64), rows = band rows between gradient and residual per cell (one upwind
+# value per face: about 1.5 faces per triangle and 2 per tetrahedron; with a
+# fixed launch shape the stored gradient's components), rec = bytes of one
+# sweep record (per direction and cell). Per band*direction*cell update unless
+# noted:
+#   gradient  read e, write the rows                  (1 + rows) s
+#   residual  read e and the rows, write R            (2 + rows) s
 #   sweep     read R, write the corrections, read the
 #             level records once per band             2 s + rec / nb
 #   moments   read e and the corrections, write e     3 s
 #   pcg       (per launch) the macro system and three vectors, read once:
 #             nnz (8 B value + 4 B column) + nc (b, x in, x out, diagonal: 32 B; order: 4 B)
-def kernel_algorithmic_bytes(name: str, s: int, dim: int, nb: int, nd: int, nc: int, nnz: int):
+def kernel_algorithmic_bytes(name: str, s: int, rows: float, nb: int, nd: int, nc: int, nnz: int):
     rec = 48 if s == 4 else 64
-    per_update = {"gradient": (1 + dim) * s, "residual": (2 + dim) * s, "sweep": 2 * s + rec / nb,
+    per_update = {"gradient": (1 + rows) * s, "residual": (2 + rows) * s, "sweep": 2 * s + rec / nb,
                   "moments": 3 * s}
     if name in per_update:
         return per_update[name] * nb * nd * nc
@@ -168,6 +171,13 @@ def macro_nnz(deck) -> int:
     right-hand side)."""
     m = deck.mesh
     return m.n_cells + sum(len(c) for c in m.cells) - len(m.edges)
+
+
+def face_rows(deck) -> float:
+    """Faces per cell (a cell has as many as vertices, in triangles, quads and
+    tetrahedra; an interior face is shared by two cells)."""
+    m = deck.mesh
+    return (sum(len(c) for c in m.cells) + len(m.edges)) / 2 / m.n_cells
 
 
 def ranks_reduce(value: float, op: str, world: int, device) -> float:
@@ -270,13 +280,15 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     total_ms = sum(v["ms"] for v in kern.values())
     dim = 2 if deck.mesh.nodes.shape[1] == 2 else 3
     nnz = macro_nnz(deck)
+    # the face-value path (residual_form 9) or gradient arrays
+    rows = face_rows(deck) if st.get("residual_form") == 9 else dim
     traffic_per_update = NCU_TRAFFIC_PER_UPDATE.get((args.workload, args.precision), {})
 
     def kernel_roofline(name):
         k = kern[name]
         per_launch_ms = k["ms"] / k["launches"]
         launches_per_step = k["launches"] / args.steps
-        alg = kernel_algorithmic_bytes(name, s_bytes, dim, nb, nd, nc, nnz)
+        alg = kernel_algorithmic_bytes(name, s_bytes, rows, nb, nd, nc, nnz)
         if alg and name in ("gradient", "residual", "sweep", "moments"):
             alg = alg / launches_per_step  # direction batches: one launch covers a batch
         achieved = alg / (per_launch_ms * 1e-3) / 1e9 if alg else None
