@@ -4254,8 +4254,8 @@ bool Solver::face_path() const {
 }
 
 // Cells per block: 32 in 2D and in the 3D FP32 form, 24 in the 3D FP64 form
-// (two CTAs per SM: its stencil entries are 32 bytes), fewer where a block's
-// tile does not fit in shared memory. Pieces and lanes per cell: 4 lanes of
+// (its stencil entries are 32 bytes), fewer where the tiles of two blocks do
+// not fit on an SM. Pieces and lanes per cell: 4 lanes of
 // 2 pieces in 2D FP32 and 8 of 2 in 2D FP64 (one stencil entry serves two
 // row loads), 8 of 1 in 3D (a wider slab would leave one CTA per SM).
 template <typename S, int DIM>
@@ -4263,15 +4263,32 @@ Error Solver::face_shape() {
     if (fshape_built_) return {0, ""};
     fshape_built_ = true;
     cudaStream_t s = cfg.stream;
-    const int best = DIM == 3 && sizeof(S) == 8 ? 24 : 32;
-    for (int B : {best, 16, 8}) {
+    // The widest block of which two fit on an SM (227 KB, 1 KB of it per block
+    // for the system), else the widest that fits at all: its shared memory is
+    // the mesh's largest union, so a width that pairs on one mesh may not on
+    // the next. 1.92 million tetrahedra x 40 bands x 64 directions (FP32): 32
+    // cells, one block per SM 126.9 ms; 28 cells, two 100.6; 24 104.7; 16 126.4.
+    constexpr int W = kFaceW<S, DIM>, best = DIM == 3 && sizeof(S) == 8 ? 24 : 32, step = 32 / W;
+    auto smem_of = [&](const GradTiles &t, int B) {
+        return ((size_t)t.qmax + 4 * B) * sizeof(FaceW<S, DIM>) +
+               (size_t)t.umax * (W * kFaceNP<DIM> * 16 + sizeof(int));
+    };
+    int width = 0;
+    GradTiles pick;
+    for (int B = best; B >= (pick.B ? 16 : 8) && width == 0; B -= B > 16 ? step : 8) {
         GradTiles t;
         if (build_grad_tiles(mesh, B, t).code) continue;
+        const size_t smem = smem_of(t, B);
+        const bool pairs = smem <= 227 * 1024 / 2 - 1024;
+        if (pairs || (B <= 16 && pick.B == 0 && smem <= 220 * 1024)) width = B;
+        if (width || (pick.B == 0 && smem <= 220 * 1024)) pick = std::move(t);
+    }
+    if (pick.B > 0) {
+        const GradTiles &t = pick;
+        const int B = t.B;
         FaceShape f;
-        f.threads = B * kFaceW<S, DIM>;
-        f.smem = ((size_t)t.qmax + 4 * B) * sizeof(FaceW<S, DIM>) +
-                 (size_t)t.umax * (kFaceW<S, DIM> * kFaceNP<DIM> * 16 + sizeof(int));
-        if (f.smem > 220 * 1024) continue;
+        f.threads = B * W;
+        f.smem = smem_of(t, B);
         if (index_checks_enabled()) {
             long long checked = 0;
             Error ce = check_tiles(mesh, &t, nullptr, checked);
@@ -4287,7 +4304,6 @@ Error Solver::face_shape() {
         CUDA_TRY(cudaFuncSetAttribute(k_grad_face<S, DIM, kFaceW<S, DIM>, kFaceNP<DIM>>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         fshape_ = f;
-        break;
     }
     return {0, ""};
 }
