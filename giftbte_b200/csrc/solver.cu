@@ -1969,7 +1969,7 @@ __global__ void k_remacro(DMesh m, const double *__restrict__ Th, const double *
 // faces x 20 bands x 32 directions 30 -> 19 us.
 constexpr int kWallSlots = 8, kWallBatch = 8;
 template <bool MOM>
-__global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nws, const int *__restrict__ wall_side,
+__global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw, const int *__restrict__ wall_side,
                                                const double *__restrict__ wtab, const double *__restrict__ dif_w,
                                                const int *__restrict__ spec_src, const double *__restrict__ snap,
                                                const double *__restrict__ ovr, double *__restrict__ dsum, double *eb,
@@ -1984,7 +1984,7 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
         __syncthreads();
     }
     const int lw = threadIdx.x / nb, b = threadIdx.x % nb, w = blockIdx.x * cpb + lw;
-    if (lw < cpb && w < nws) {
+    if (lw < cpb && w < nw) {
         const int s = wall_side[w], c = m.bs_cell[s], k = m.bs_cf[s], ib = s >> 1, type = m.b_type[ib];
         const int mo = mat_off(p, c);
         const double nx = m.cf_nx[k], ny = m.cf_ny[k], nz = m.cf_nz[k], vm = p.vmag[mo + b], Cb = p.C[mo + b];
@@ -2076,7 +2076,7 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
         __syncthreads();
         for (int t = threadIdx.x; t < cpb * kWallSlots; t += blockDim.x) {
             const int i = t / kWallSlots, j = t % kWallSlots, ww = blockIdx.x * cpb + i;
-            if (ww >= nws) continue;
+            if (ww >= nw) continue;
             double sum = 0;
             for (int bb = 0; bb < nb; bb++) sum += part[((size_t)i * nb + bb) * kWallSlots + j];
             const int s = wall_side[ww];
@@ -3663,17 +3663,30 @@ Error Solver::init(const FlatMesh &m, const Bands &b, const Angles &a, const std
         bTF_ = up_d(bT);
         bF_dir_ = up_i(dir);
     }
-    // wall slot of every wall face of a cell (-1 on interior faces)
+    // wall slot of every wall face of a cell (-1 on interior faces), and the
+    // wall sides: the one each slot's face refers to, in slot order, then the
+    // sides that name a face again (a boundary element given twice, or a tag
+    // in two rows of the boundary table), which periodic partners and node
+    // values may refer to
     {
-        std::vector<int> gw(mesh.ncf(), -1), ws;
+        std::vector<int> gw(mesh.ncf(), -1), ws, slot;
         for (int k = 0; k < mesh.ncf(); k++)
             if (mesh.cf_bound[k] >= 0) {
                 gw[k] = (int)ws.size();
+                slot.push_back(gw[k]);
                 ws.push_back(mesh.cf_bside[k]);
             }
         n_wall_slots_ = (int)ws.size();
+        for (int sd = 0; sd < mesh.nbs(); sd++) {
+            const int k = mesh.bs_cell[sd] < 0 ? -1 : mesh.bs_cf[sd];
+            if (k < 0 || mesh.cf_bside[k] == sd) continue;
+            slot.push_back(gw[k]);
+            ws.push_back(sd);
+        }
+        n_walls_ = (int)ws.size();
         cf_gw_ = up_i(gw);
         wall_side_ = up_i(ws);
+        wall_slot_ = up_i(slot);
     }
     if (!ok) return {-6, "device allocation or upload failed"};
     Error e = alloc_all();
@@ -4350,21 +4363,21 @@ void Solver::launch_moments(S *eps, bool apply, int d0, int nbt, bool accumulate
 // the wall kernel, with or without the moments (outside the solve's stages
 // it only refreshes the incoming values)
 void Solver::launch_walls(bool moments) {
-    if (n_wall_slots_ == 0) return;
+    if (n_walls_ == 0) return;
     const int nb = bands.nb, nd = ang.nd;
     cudaStream_t s = cfg.stream;
     if (need_snapshot_)
         cudaMemcpyAsync(eb_snap_, eb_, (size_t)nd * mesh.nbs() * nb * 8, cudaMemcpyDeviceToDevice, s);
     // walls per block: 256 threads' worth, fewer where that leaves SMs without a block
-    const int cpb = std::max(1, std::min(256 / nb, (n_wall_slots_ + 147) / 148));
-    const int grid = (n_wall_slots_ + cpb - 1) / cpb, thr = (cpb * nb + 31) / 32 * 32;
+    const int cpb = std::max(1, std::min(256 / nb, (n_walls_ + 147) / 148));
+    const int grid = (n_walls_ + cpb - 1) / cpb, thr = (cpb * nb + 31) / 32 * 32;
     const double *snap = need_snapshot_ ? eb_snap_ : nullptr;
     if (moments) {
         const size_t smem = ((size_t)nd * kWTab + (size_t)thr * kWallSlots) * sizeof(double);
-        k_walls<true><<<grid, thr, smem, s>>>(dm_, dp_, cpb, n_wall_slots_, wall_side_, wtab_, dif_w_, spec_src_, snap,
+        k_walls<true><<<grid, thr, smem, s>>>(dm_, dp_, cpb, n_walls_, wall_side_, wtab_, dif_w_, spec_src_, snap,
                                               bTovr_, dsum_, eb_, Ths_, Qs_, bTm_);
     } else {
-        k_walls<false><<<grid, thr, 0, s>>>(dm_, dp_, cpb, n_wall_slots_, wall_side_, wtab_, dif_w_, spec_src_, snap,
+        k_walls<false><<<grid, thr, 0, s>>>(dm_, dp_, cpb, n_walls_, wall_side_, wtab_, dif_w_, spec_src_, snap,
                                             bTovr_, dsum_, eb_, Ths_, Qs_, bTm_);
     }
 }
@@ -4536,10 +4549,10 @@ Error Solver::solve_t(SolveStats &st) {
         if (!(face_path() && fshape_.tile.B > 0))
             GL(K_BOUND_OUT, (k_bound_out<S, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_,
                                                                                                    d0, nbt)));
-        else if (n_wall_slots_ > 0)
-            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<wall_grid((size_t)n_wall_slots_ * nb, nbt), kThreads, 0, s>>>(
-                                dm_, dp_, eps, (const S *)wall_grad_, n_wall_slots_, wall_side_, Tbase_, gTb_, eb_, d0,
-                                nbt)));
+        else if (n_walls_ > 0)
+            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<wall_grid((size_t)n_walls_ * nb, nbt), kThreads, 0, s>>>(
+                                dm_, dp_, eps, (const S *)wall_grad_, n_wall_slots_, n_walls_, wall_side_, wall_slot_,
+                                Tbase_, gTb_, eb_, d0, nbt)));
     };
     // LSQ gradient, 4 bands and grad_dg directions per thread (options.gradient_dirs,
     // or timed on the first outer iteration: gtune)
@@ -5296,9 +5309,10 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
     auto bound_out = [&](int d0, int nbt) {
         if (!faces)
             k_bound_out<double, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0, nbt);
-        else if (n_wall_slots_ > 0)
-            k_bound_out_w<double, DIM><<<wall_grid((size_t)n_wall_slots_ * nb, nbt), kThreads, 0, s>>>(
-                dm_, dp_, eps, (const double *)wall_grad_, n_wall_slots_, wall_side_, Tbase_, gTb_, eb_, d0, nbt);
+        else if (n_walls_ > 0)
+            k_bound_out_w<double, DIM><<<wall_grid((size_t)n_walls_ * nb, nbt), kThreads, 0, s>>>(
+                dm_, dp_, eps, (const double *)wall_grad_, n_wall_slots_, n_walls_, wall_side_, wall_slot_, Tbase_, gTb_,
+                eb_, d0, nbt);
     };
     for (int d0 = 0; d0 < nd; d0 += ndb) {
         const int nbt = std::min(ndb, nd - d0);

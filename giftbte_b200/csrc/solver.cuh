@@ -250,8 +250,10 @@ private:
     void *wall_grad_ = nullptr;
     unsigned char *face_mask_ = nullptr;
     int *cf_gw_ = nullptr;
-    int *wall_side_ = nullptr;  // [n_wall_slots_] boundary side of every wall slot
     int n_wall_slots_ = 0;
+    // [n_walls_] every boundary side that has a cell, and its face's wall slot
+    int *wall_side_ = nullptr, *wall_slot_ = nullptr;
+    int n_walls_ = 0;
     double *Tbase_ = nullptr, *gTb_ = nullptr;
     double *Bflux_ = nullptr;  // [nd][nc] base-field face flux sums of the residual
     double *eb_ = nullptr, *eb_snap_ = nullptr;
