@@ -90,6 +90,11 @@ struct FlatMesh {
     std::vector<int> cf_v;  // [ncf*3] face vertices (third = -1 in 2D)
     // global faces (Element_Faces order, BTEMesh.cpp:987-1021)
     std::vector<int> f_cell0, f_cf0, f_cell1, f_cf1, f_bound;
+    // every interior face belongs to exactly two cell faces, which name it in
+    // cf_face (not where two cells share two faces, as a concave quadrilateral
+    // and the cell in its notch do: the list then follows the cells, not the
+    // faces)
+    bool faces_paired = false;
     // vertex-neighbour least-squares stencil (StaticBTESynthetic.cpp:453-465,
     // 967-1025); weights already include the 1/ScaleX factors
     std::vector<int> nbr_ptr, nbr_idx;

@@ -391,6 +391,14 @@ Error build_flat_mesh(const RawMesh &raw, const BCs &bcs, const Bands &bands, Fl
         if (m.b_connect[ib] < 0) return {-7, "periodic boundary tag " + std::to_string(tags[b_row[ib]]) + " has no partner"};
     }
     // global face list
+    auto same_vertices = [&](int k, int q) {
+        for (int t = 0; t < fnv; t++) {
+            bool in = false;
+            for (int u = 0; u < fnv; u++) in = in || m.cf_v[3 * k + t] == m.cf_v[3 * q + u];
+            if (!in) return false;
+        }
+        return true;
+    };
     {
         std::vector<char> done(ncf, 0);
         for (int c = 0; c < nc; c++)
@@ -410,10 +418,13 @@ Error build_flat_mesh(const RawMesh &raw, const BCs &bcs, const Bands &bands, Fl
                             m.cf_face[q] = f;
                             // one centre per face: the two cells list its
                             // vertices in different orders, which rounds a
-                            // triangle's mean differently
-                            m.cf_fx[q] = m.cf_fx[k];
-                            m.cf_fy[q] = m.cf_fy[k];
-                            m.cf_fz[q] = m.cf_fz[k];
+                            // triangle's mean differently (an edge's is the
+                            // same either way)
+                            if (dim == 3 && same_vertices(k, q)) {
+                                m.cf_fx[q] = m.cf_fx[k];
+                                m.cf_fy[q] = m.cf_fy[k];
+                                m.cf_fz[q] = m.cf_fz[k];
+                            }
                         }
                 }
                 m.f_cell0.push_back(c);
@@ -422,6 +433,15 @@ Error build_flat_mesh(const RawMesh &raw, const BCs &bcs, const Bands &bands, Fl
                 m.f_cf1.push_back(k1);
                 m.f_bound.push_back(m.cf_bound[k]);
             }
+        std::vector<int> sides(m.nf(), 0);
+        for (int k = 0; k < ncf; k++) sides[m.cf_face[k]]++;
+        m.faces_paired = true;
+        for (int f = 0; f < m.nf(); f++) {
+            if (m.f_bound[f] != -1) continue;
+            const int k = m.f_cf0[f], q = m.f_cf1[f];
+            if (!(sides[f] == 2 && q >= 0 && m.cf_face[k] == f && m.cf_face[q] == f && same_vertices(k, q)))
+                m.faces_paired = false;
+        }
     }
     // vertex-neighbour LSQ stencil: every cell around each of the cell's
     // vertices, in vertex order then node-to-cell order, once each, same

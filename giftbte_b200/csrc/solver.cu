@@ -4257,12 +4257,14 @@ constexpr int kFaceNP = DIM == 2 ? 2 : 1;
 // The face-value path serves the second-order scheme without the limiter
 // when a band row is a whole number of 16-byte pieces; a launch shape fixed
 // by the caller (options.gradient_dirs, residual_form) keeps the
-// gradient-array kernels. FP32 rows of other lengths stay on the one-band
-// kernels, whose face sums are formed in FP64.
+// gradient-array kernels, and so does a mesh whose cell faces do not pair up
+// (two cells that share two faces: a face would have two writers or none).
+// FP32 rows of other lengths stay on the one-band kernels, whose face sums
+// are formed in FP64.
 bool Solver::face_path() const {
     const size_t s = cfg.precision == 1 ? sizeof(float) : sizeof(double);
     if ((size_t)bands.nb * bands.nmat * 24 > 40 * 1024) return false;  // the band constants are staged per CTA
-    return cfg.order == 2 && !cfg.use_limiter && cfg.gradient_dirs == 0 && cfg.residual_form == 0 &&
+    return mesh.faces_paired && cfg.order == 2 && !cfg.use_limiter && cfg.gradient_dirs == 0 && cfg.residual_form == 0 &&
            bands.nb * s % 16 == 0 && (size_t)std::max(mesh.nc, mesh.nf()) * bands.nb < ((size_t)1 << 31);
 }
 
