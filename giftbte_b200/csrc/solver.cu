@@ -4070,7 +4070,9 @@ Error Solver::cg_plan(const std::vector<int> &ptr, const std::vector<int> &idx, 
     const size_t line = 8 * ((size_t)8 * nrmax + hmax + 256 + (size_t)4 * NA + kCgAgg + (size_t)K * nrmax + smax) +
                         4 * ((size_t)K * nrmax + smax + kCgAgg + 1);
     if (std::max(smem, line) > (size_t)max_smem || nrmax + hmax > 65535) return {0, ""};
-    CUDA_TRY(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the limit belongs to the kernel, not to the handle: never lowered to
+    // this plan's own size, which another handle's larger plan would miss)
+    CUDA_TRY(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     CUDA_TRY(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3(C);
@@ -6617,7 +6619,8 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
     const int sthreads = std::max(nbc, (256 / nbc) * nbc);
     const int last = nb - (chunks - 1) * nbc;
     const int rvec = ((nbc * 8) % 16 == 0 && (nb * 8) % 16 == 0 && (last * 8) % 16 == 0) ? 1 : 0;
-    CUDA_TRY(cudaFuncSetAttribute(k_sweep<double, LOOK, LCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the limit belongs to the kernel, not to the handle: every caller sets the same)
+    CUDA_TRY(cudaFuncSetAttribute(k_sweep<double, LOOK, LCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     const int N = last_inner_;
     long long cg_its = 0;
     // warm starts of the reverse Picard solves: each step's solution of the
