@@ -313,7 +313,6 @@ __global__ void __launch_bounds__(256, DIM == 2 ? 4 : 2)
 // gives the same bits.
 __device__ __forceinline__ float add_face(float acc, float a, float y) { return __fadd_rn(acc, __fmul_rn(a, y)); }
 __device__ __forceinline__ double add_face(double acc, double a, double y) { return acc + a * y; }
-constexpr int kResDirs = 8;
 template <typename S, int DIM>
 __global__ void __launch_bounds__(256, 3) k_resid_face(DMesh m, DPhys p, int cpb, const S *__restrict__ eps,
                                                        const S *__restrict__ F,

@@ -226,6 +226,18 @@ struct GradTiles {
 };
 Error build_grad_tiles(const FlatMesh &m, int B, GradTiles &out);
 
+// Shared memory of a CTA of the face-value residual: the band constants of
+// every material and the coefficients of its cells and kResDirs directions.
+// nb * size is a multiple of 16 (size: bytes of a stored intensity).
+constexpr int kResDirs = 8;
+inline int resid_face_cells(int nb, size_t size) {
+    const int ppd = (int)(nb * size / 16);
+    return ppd > 256 ? 1 : 256 / ppd < 128 ? 256 / ppd : 128;
+}
+inline size_t resid_face_smem(int nb, int nmat, size_t size) {
+    return (size_t)nb * nmat * (16 + size) + (size_t)kResDirs * resid_face_cells(nb, size) * 4 * size;
+}
+
 // Tiles of the shared-memory residual: the same blocks, each union its own
 // cells then its cells' interior face neighbours outside it (ascending);
 // floc[k] is the union index of face slot k's neighbour (0xFFFF on walls).

@@ -4260,14 +4260,16 @@ constexpr int kFaceNP = DIM == 2 ? 2 : 1;
 // when a band row is a whole number of 16-byte pieces; a launch shape fixed
 // by the caller (options.gradient_dirs, residual_form) keeps the
 // gradient-array kernels, and so does a mesh whose cell faces do not pair up
-// (two cells that share two faces: a face would have two writers or none).
+// (two cells that share two faces: a face would have two writers or none) and
+// a band table that the residual cannot stage in the 48 KB of shared memory a
+// kernel has by default (FP64, 4 bands: 171 materials).
 // FP32 rows of other lengths stay on the one-band kernels, whose face sums
 // are formed in FP64.
 bool Solver::face_path() const {
     const size_t s = cfg.precision == 1 ? sizeof(float) : sizeof(double);
-    if ((size_t)bands.nb * bands.nmat * 24 > 40 * 1024) return false;  // the band constants are staged per CTA
     return mesh.faces_paired && cfg.order == 2 && !cfg.use_limiter && cfg.gradient_dirs == 0 && cfg.residual_form == 0 &&
-           bands.nb * s % 16 == 0 && (size_t)std::max(mesh.nc, mesh.nf()) * bands.nb < ((size_t)1 << 31);
+           bands.nb * s % 16 == 0 && resid_face_smem(bands.nb, bands.nmat, s) <= 48 * 1024 &&
+           (size_t)std::max(mesh.nc, mesh.nf()) * bands.nb < ((size_t)1 << 31);
 }
 
 // Cells per block: 32 in 2D and in the 3D FP32 form, 24 in the 3D FP64 form
@@ -4388,10 +4390,9 @@ void Solver::launch_walls(bool moments) {
 
 template <typename S, int DIM>
 cudaError_t Solver::launch_resid_face(const S *eps, const double *Told, int d0, int nbt) {
-    const int nb = bands.nb, ppd = nb / kPieceBands<S>;
-    const int cpb = std::max(1, std::min(128, 256 / ppd));
+    const int nb = bands.nb, ppd = nb / kPieceBands<S>, cpb = resid_face_cells(nb, sizeof(S));
     const dim3 grid((mesh.nc + cpb - 1) / cpb, (nbt + kResDirs - 1) / kResDirs);
-    const size_t smem = (size_t)nb * bands.nmat * (16 + sizeof(S)) + (size_t)kResDirs * cpb * 4 * sizeof(S);
+    const size_t smem = resid_face_smem(nb, bands.nmat, sizeof(S));
     k_resid_face<S, DIM><<<grid, ((cpb * ppd + 31) / 32) * 32, smem, cfg.stream>>>(
         dm_, dp_, cpb, eps, (const S *)grad_, face_mask_, Tbase_, Bflux_, Told, eb_, pos_of_, (S *)res_, d0, nbt);
     return cudaGetLastError();
@@ -5380,7 +5381,7 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
             ev.gd0 = d0;
             if (faces) {
                 CUDA_TRY((launch_grad_face<double, DIM>(eps, d0, nbt)));
-                const int ppd = nb / kPieceBands<double>, cpb = std::max(1, std::min(128, 256 / ppd));
+                const int ppd = nb / kPieceBands<double>, cpb = resid_face_cells(nb, sizeof(double));
                 const dim3 grid((nc + cpb - 1) / cpb, (nbt + kResDirs - 1) / kResDirs);
                 k_tr_step_face<DIM><<<grid, (cpb * ppd + 31) / 32 * 32, (size_t)kResDirs * cpb * 4 * 8, s>>>(
                     dm_, dp_, cpb, eps, g, face_mask_, T_, eb_, dt, d0, nbt);
