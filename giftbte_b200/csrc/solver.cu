@@ -1946,8 +1946,8 @@ __global__ void k_remacro(DMesh m, const double *__restrict__ Th, const double *
 }
 
 
-// Everything that one iteration needs of the walls, a thread per (wall side,
-// band) walking the directions of eb[d][s][b] twice.
+// Everything that one iteration needs of the walls, `split` threads per (wall
+// side, band), each walking its share of the directions of eb[d][s][b] twice.
 //  First pass, over the values before the refresh (as the reference evaluates
 //  its face gradients inside the pair loop): with MOM the moments Ths, Qs of
 //  the synthetic source; the diffuse re-emission sum of types 2, 5, 6 into
@@ -1958,18 +1958,20 @@ __global__ void k_remacro(DMesh m, const double *__restrict__ Th, const double *
 //  so no thread sees another's writes. With MOM the lattice temperature of
 //  the refreshed values, bTm, with the periodic overrides.
 // Band sums are formed in shared memory in band order, as in k_moments.
-// blockDim = cpb * nb (rounded up to a warp). Geometry and band constants are
-// formed once per thread, where four kernels with a thread per (direction,
+// blockDim = cpb * nb * split (rounded up to a warp). Geometry and band
+// constants are formed once per thread, where four kernels with a thread per (direction,
 // side, band) or a warp per side formed them per value, divisions included:
 // 4,800 wall faces x 40 bands x 128 directions 0.79 -> 0.25 ms.
 // With few walls it is bound by the latency of its own chain over the
 // directions: the second pass loads kWallBatch values before it stores any
 // (the compiler cannot move a load over the stores to eb), and blocks hold
 // fewer walls so that every SM has one (launch_walls): the refresh of 240 wall
-// faces x 20 bands x 32 directions 30 -> 19 us.
+// faces x 20 bands x 32 directions 30 -> 19 us. Where a block would still have
+// few threads and many directions (few bands), the directions are split.
 constexpr int kWallSlots = 8, kWallBatch = 8;
 template <bool MOM>
-__global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw, const int *__restrict__ wall_side,
+__global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int split, int nw,
+                                               const int *__restrict__ wall_side,
                                                const double *__restrict__ wtab, const double *__restrict__ dif_w,
                                                const int *__restrict__ spec_src, const double *__restrict__ snap,
                                                const double *__restrict__ ovr, double *__restrict__ dsum, double *eb,
@@ -1979,13 +1981,16 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
     double *wt = sm_dyn;  // [nd][kWTab]
     const int nb = p.nb, nd = p.nd;
     double *part = sm_dyn + (size_t)nd * kWTab;  // [blockDim][kWallSlots]
+    __shared__ double sums[2][256];
     if constexpr (MOM) {
         for (int i = threadIdx.x; i < nd * kWTab; i += blockDim.x) wt[i] = wtab[i];
         __syncthreads();
     }
-    const int lw = threadIdx.x / nb, b = threadIdx.x % nb, w = blockIdx.x * cpb + lw;
-    if (lw < cpb && w < nw) {
-        const int s = wall_side[w], c = m.bs_cell[s], k = m.bs_cf[s], ib = s >> 1, type = m.b_type[ib];
+    const int rows = cpb * nb, part_of = threadIdx.x / rows, r = threadIdx.x - part_of * rows, lw = r / nb,
+              b = r - lw * nb, w = blockIdx.x * cpb + lw;
+    const bool on = part_of < split && w < nw;
+    {
+        const int s = wall_side[on ? w : 0], c = m.bs_cell[s], k = m.bs_cf[s], ib = s >> 1, type = m.b_type[ib];
         const int mo = mat_off(p, c);
         const double nx = m.cf_nx[k], ny = m.cf_ny[k], nz = m.cf_nz[k], vm = p.vmag[mo + b], Cb = p.C[mo + b];
         const double hr = p.hr[mo + b];
@@ -1994,10 +1999,13 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
         const double *dw = dif_w + (size_t)s * nd;
         const bool dif = type == 2 || type == 6;
         auto incoming = [&](int d) { return vm * p.sx[d] * nx + vm * p.sy[d] * ny + vm * p.sz[d] * nz < 0; };
+        // this thread's directions
+        const int share = (nd + split - 1) / split, q0 = on ? min(part_of * share, nd) : 0,
+                  q1 = on ? min(q0 + share, nd) : 0;
         double a[7] = {0, 0, 0, 0, 0, 0, 0}, acc = 0, a1 = 0, a2 = 0, lat = 0;
         // (the refresh alone needs the pass only for a re-emission sum)
 #pragma unroll 8
-        for (int d = 0; d < (MOM || dif || type == 5 ? nd : 0); d++) {
+        for (int d = q0; d < (MOM || dif || type == 5 ? q1 : q0); d++) {
             const double x = row[d * str];
             if constexpr (MOM) {
                 const double *q = wt + kWTab * d;
@@ -2016,6 +2024,14 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
                 else if (wq < 0) a2 -= wq * eb[d * str + (size_t)(s ^ 1) * nb + b];
             }
         }
+        if (split > 1) {  // the re-emission sums over all directions
+            sums[0][threadIdx.x] = type == 5 ? a1 : acc;
+            sums[1][threadIdx.x] = a2;
+            __syncthreads();
+            acc = a1 = a2 = 0;
+            for (int l = 0; l < split; l++) acc += sums[0][l * rows + r], a2 += sums[1][l * rows + r];
+            a1 = acc;
+        }
         if (type == 5) {
             // interface: (1 - t) (|v_1| <e_out,1> + |v_2| <e_out,2>) / |v_1|,
             // side 1 this one, side 2 the other, t this side's transmissivity
@@ -2023,7 +2039,7 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
             const double tr = m.bs_trans[(size_t)s * nb + b];
             acc = (vm * a1 * (1 - tr) + v2 * a2 * (1 - tr)) / vm;
         }
-        if (dif || type == 5) dsum[(size_t)s * nb + b] = acc;
+        if (on && part_of == 0 && (dif || type == 5)) dsum[(size_t)s * nb + b] = acc;
         if (hr != 0) {
             const double bT = m.b_T[ib];
             const int cb = type < 0 ? m.b_connect[ib] : 0;
@@ -2032,13 +2048,13 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
             const double *from = (snap && type == 3 ? snap : eb) + (size_t)s * nb + b;
             const double *src = type < 0 ? partner : from;
             const bool cst = type == 1 || type == 2 || type == 5, far = type == 3 || type == 6 || type < 0;
-            for (int d0 = 0; (cst || far) && d0 < nd; d0 += kWallBatch) {
+            for (int d0 = q0; (cst || far) && d0 < q1; d0 += kWallBatch) {
                 double x[kWallBatch];
                 unsigned in = 0;
 #pragma unroll
                 for (int i = 0; i < kWallBatch; i++) {
                     const int d = d0 + i;
-                    if (d >= nd || !incoming(d)) continue;
+                    if (d >= q1 || !incoming(d)) continue;
                     in |= 1u << i;
                     if (far) x[i] = src[(type < 0 ? d : spec_src[(size_t)s * nd + d]) * str];
                 }
@@ -2078,7 +2094,8 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int nw
             const int i = t / kWallSlots, j = t % kWallSlots, ww = blockIdx.x * cpb + i;
             if (ww >= nw) continue;
             double sum = 0;
-            for (int bb = 0; bb < nb; bb++) sum += part[((size_t)i * nb + bb) * kWallSlots + j];
+            for (int bb = 0; bb < nb; bb++)
+                for (int l = 0; l < split; l++) sum += part[((size_t)l * rows + i * nb + bb) * kWallSlots + j];
             const int s = wall_side[ww];
             if (j == 0) {
                 Ths[s] = (p.mat ? p.kap[p.mat[m.bs_cell[s]]] : p.kappa) * sum;
@@ -4376,14 +4393,19 @@ void Solver::launch_walls(bool moments) {
         cudaMemcpyAsync(eb_snap_, eb_, (size_t)nd * mesh.nbs() * nb * 8, cudaMemcpyDeviceToDevice, s);
     // walls per block: 256 threads' worth, fewer where that leaves SMs without a block
     const int cpb = std::max(1, std::min(256 / nb, (n_walls_ + 147) / 148));
-    const int grid = (n_walls_ + cpb - 1) / cpb, thr = (cpb * nb + 31) / 32 * 32;
+    // threads per (wall, band): as many as the block still holds, of at least
+    // one batch of directions each (gray square, 160 walls, 1024 directions:
+    // five iterations 10.9 -> 6.2 ms; 60 specular and periodic walls x 2 bands
+    // x 256 directions, the refresh alone: 26 -> 11 us)
+    const int split = std::max(1, std::min(256 / (cpb * nb), nd / kWallBatch));
+    const int grid = (n_walls_ + cpb - 1) / cpb, thr = (cpb * nb * split + 31) / 32 * 32;
     const double *snap = need_snapshot_ ? eb_snap_ : nullptr;
     if (moments) {
         const size_t smem = ((size_t)nd * kWTab + (size_t)thr * kWallSlots) * sizeof(double);
-        k_walls<true><<<grid, thr, smem, s>>>(dm_, dp_, cpb, n_walls_, wall_side_, wtab_, dif_w_, spec_src_, snap,
+        k_walls<true><<<grid, thr, smem, s>>>(dm_, dp_, cpb, split, n_walls_, wall_side_, wtab_, dif_w_, spec_src_, snap,
                                               bTovr_, dsum_, eb_, Ths_, Qs_, bTm_);
     } else {
-        k_walls<false><<<grid, thr, 0, s>>>(dm_, dp_, cpb, n_walls_, wall_side_, wtab_, dif_w_, spec_src_, snap,
+        k_walls<false><<<grid, thr, 0, s>>>(dm_, dp_, cpb, split, n_walls_, wall_side_, wtab_, dif_w_, spec_src_, snap,
                                             bTovr_, dsum_, eb_, Ths_, Qs_, bTm_);
     }
 }
