@@ -6353,37 +6353,42 @@ __global__ void k_adj_u(DMesh m, const double *__restrict__ Q, const double *__r
     U[c] = acc + m.heat[c] * m.vol[c];
 }
 
-// Gradient assembly over cells, a thread per (cell, band) walking the
-// directions (blockDim = cpb * nb, rounded up to a warp).
+// Gradient assembly over cells, `split` threads per (cell, band), each walking
+// its share of the directions (blockDim = cpb * nb * split, rounded up to a
+// warp; assemble_shape).
 // Gamma = lam (e - C_b T*) gives the residual's tau and s_c derivatives; the
 // tensor moment's tau derivative is v_b^2 (w s s^T e) : Qbar. Sums over the
 // block's cells per band and over a cell's bands go through shared memory,
 // one atomic per band and block into g_tau. Bound by reading lam and e; a
 // warp per cell with lanes over (direction, band) and a shared-memory FP64
-// atomic per value: 54 -> 27 us on 6,488 triangles x 20 bands x 32
+// atomic per value: 57 -> 27 us on 6,488 triangles x 20 bands x 32
 // directions.
-__global__ void __launch_bounds__(256) k_adj_assemble(DMesh m, DPhys p, int cpb, const double *__restrict__ lam,
+__global__ void __launch_bounds__(256) k_adj_assemble(DMesh m, DPhys p, int cpb, int split,
+                                                      const double *__restrict__ lam,
                                                       const double *__restrict__ eps, const double *__restrict__ T,
                                                       const double *__restrict__ Qbar, double *g_cell, double *g_tau) {
     __shared__ double sg[256], st[256];
-    const int nb = p.nb, ci = threadIdx.x / nb, b = threadIdx.x % nb, c = blockIdx.x * cpb + ci;
+    const int nb = p.nb, rows = cpb * nb, part = threadIdx.x / rows, r = threadIdx.x - part * rows, ci = r / nb,
+              b = r - ci * nb, c = blockIdx.x * cpb + ci;
     double gs = 0, ts = 0;
-    if (ci < cpb && c < m.nc) {
+    if (part < split && c < m.nc) {
         const double ct = p.C[b] * T[c], f = p.tau[b] * p.vmag[b] * p.vmag[b];
         const double *q = Qbar + 6 * (size_t)c;
         const double q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];
         const bool syn = p.hr[b] > 0;
         const size_t row = (size_t)m.nc * nb;
-        const double *ep = eps + (size_t)c * nb + b, *lp = lam + (size_t)c * nb + b;
+        const int share = (p.nd + split - 1) / split, first = min(part * share, p.nd), n = min(share, p.nd - first);
+        const double *ep = eps + first * row + (size_t)c * nb + b, *lp = lam + first * row + (size_t)c * nb + b;
+        const double *w = p.w + first, *x = p.sx + first, *y = p.sy + first, *z = p.sz + first;
 #pragma unroll 8
-        for (int d = 0; d < p.nd; d++) {
+        for (int d = 0; d < n; d++) {
             const double e = ep[d * row];
             const double G = lp[d * row] * (e - ct);
             gs += G;
             double tb = G;  // d/d(ln tau_b) of the residual
             if (syn) {
-                const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
-                tb += f * p.w[d] * e * (q0 * sx * sx + q1 * sx * sy + q2 * sx * sz + q3 * sy * sy + q4 * sy * sz + q5 * sz * sz);
+                const double sx = x[d], sy = y[d], sz = z[d];
+                tb += f * w[d] * e * (q0 * sx * sx + q1 * sx * sy + q2 * sx * sz + q3 * sy * sy + q4 * sy * sz + q5 * sz * sz);
             }
             ts += tb;
         }
@@ -6391,6 +6396,11 @@ __global__ void __launch_bounds__(256) k_adj_assemble(DMesh m, DPhys p, int cpb,
     sg[threadIdx.x] = gs;
     st[threadIdx.x] = ts;
     __syncthreads();
+    if (split > 1) {  // the shares of each (cell, band)
+        if (part == 0)
+            for (int l = 1; l < split; l++) sg[r] += sg[l * rows + r], st[r] += st[l * rows + r];
+        __syncthreads();
+    }
     const int ncell = min(cpb, m.nc - (int)blockIdx.x * cpb);
     for (int i = threadIdx.x; i < nb + ncell; i += blockDim.x) {
         double sum = 0;
@@ -6406,19 +6416,20 @@ __global__ void __launch_bounds__(256) k_adj_assemble(DMesh m, DPhys p, int cpb,
 }
 
 // the tensor moment's tau derivative on wall sides, and the specularity
-// derivative of partially specular walls: a thread per (side, band) walking
-// the directions, sums as in k_adj_assemble (a warp per side with atomics per
-// value: 28.6 -> 27.3 us for 732 wall sides x 20 bands x 32 directions)
-__global__ void __launch_bounds__(256) k_adj_assemble_sides(DMesh m, DPhys p, int cpb, const double *__restrict__ eb,
+// derivative of partially specular walls: threads per (side, band) and sums
+// as in k_adj_assemble (a warp per side with atomics per value: 31 -> 19 us for
+// 732 wall sides x 20 bands x 32 directions)
+__global__ void __launch_bounds__(256) k_adj_assemble_sides(DMesh m, DPhys p, int cpb, int split, const double *__restrict__ eb,
                                                             const double *__restrict__ ebb,
                                                             const double *__restrict__ dsum,
                                                             const int *__restrict__ spec_src,
                                                             const double *__restrict__ Qsbar, double *g_tau,
                                                             double *g_bnd) {
     __shared__ double sp[256], st[256];
-    const int nb = p.nb, li = threadIdx.x / nb, b = threadIdx.x % nb, s = blockIdx.x * cpb + li;
+    const int nb = p.nb, rows = cpb * nb, part = threadIdx.x / rows, r = threadIdx.x - part * rows, li = r / nb,
+              b = r - li * nb, s = blockIdx.x * cpb + li;
     double gp = 0, ts = 0;
-    if (li < cpb && s < m.nbs && m.bs_cell[s] >= 0 && p.hr[b] > 0) {
+    if (part < split && s < m.nbs && m.bs_cell[s] >= 0 && p.hr[b] > 0) {
         const int k = m.bs_cf[s];
         const bool partial = m.b_type[s >> 1] == 6;
         const double f = p.tau[b] * p.vmag[b] * p.vmag[b];
@@ -6426,20 +6437,21 @@ __global__ void __launch_bounds__(256) k_adj_assemble_sides(DMesh m, DPhys p, in
         const double *q = Qsbar + 6 * (size_t)s;
         const double q0 = q[0], q1 = q[1], q2 = q[2], q3 = q[3], q4 = q[4], q5 = q[5];
         const size_t row = (size_t)m.nbs * nb, at = (size_t)s * nb + b;
+        const int share = (p.nd + split - 1) / split, first = part * share, end = min(first + share, p.nd);
 #pragma unroll 8
-        for (int d = 0; d < p.nd; d++) {
+        for (int d = first; d < end; d++) {
             const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
             const double x = eb[d * row + at];
             ts += f * p.w[d] * x * (q0 * sx * sx + q1 * sx * sy + q2 * sx * sz + q3 * sy * sy + q4 * sy * sz + q5 * sz * sz);
         }
         // (every load of a batch before its first use)
         const double dif = partial ? dsum[at] : 0.0;
-        for (int d0 = 0; partial && d0 < p.nd; d0 += 8) {
+        for (int d0 = first; partial && d0 < end; d0 += 8) {
             double y[8], z[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const int d = min(d0 + i, p.nd - 1);
-                const bool in = d0 + i < p.nd && p.sx[d] * nx + p.sy[d] * ny + p.sz[d] * nz < 0;
+                const bool in = d0 + i < end && p.sx[d] * nx + p.sy[d] * ny + p.sz[d] * nz < 0;
                 y[i] = eb[(in ? spec_src[(size_t)s * p.nd + d] : d) * row + at];
                 z[i] = in ? ebb[d * row + at] : 0.0;
                 if (!in) y[i] = dif;
@@ -6451,6 +6463,11 @@ __global__ void __launch_bounds__(256) k_adj_assemble_sides(DMesh m, DPhys p, in
     sp[threadIdx.x] = gp;
     st[threadIdx.x] = ts;
     __syncthreads();
+    if (split > 1) {
+        if (part == 0)
+            for (int l = 1; l < split; l++) sp[r] += sp[l * rows + r], st[r] += st[l * rows + r];
+        __syncthreads();
+    }
     const int ns = min(cpb, m.nbs - (int)blockIdx.x * cpb);
     for (int i = threadIdx.x; i < nb + ns; i += blockDim.x) {
         double sum = 0;
@@ -6745,10 +6762,26 @@ Error Solver::vjp(const double *Tbar_h, const double *qbar_h, int max_iter, doub
     const double mdim = bands.material_dim == 2 ? 2.0 : 3.0;
     auto assemble = [&](std::vector<double> &gt, std::vector<double> &gc, std::vector<double> &gb) -> Error {
         CUDA_TRY(cudaMemsetAsync(gtau, 0, (size_t)(nb + nbd) * 8, s));
-        const int cpb = std::max(1, kThreads / nb), thr = (cpb * nb + 31) / 32 * 32;
-        k_adj_assemble<<<(nc + cpb - 1) / cpb, thr, 0, s>>>(dm_, dp_, cpb, lam, eps, T_, Qbar, gcell, gtau);
-        k_adj_assemble_sides<<<(nbs + cpb - 1) / cpb, thr, 0, s>>>(dm_, dp_, cpb, eb_, ebb, dsum_, spec_src_, Qsbar,
-                                                                   gtau, gbnd);
+        // items (cells or sides) per block: 256 threads' worth, fewer where
+        // that leaves SMs without a block; then as many threads per (item,
+        // band) as the block holds, of at least eight directions each (400
+        // cells x 1 band x 256 directions: cells 140 -> 11 us, sides 223 ->
+        // 13 us)
+        struct Shape {
+            int cpb, split, grid, thr;
+        };
+        auto assemble_shape = [&](int n) {
+            Shape f;
+            f.cpb = std::max(1, std::min(kThreads / nb, (n + 147) / 148));
+            f.split = std::max(1, std::min(kThreads / (f.cpb * nb), nd / 8));
+            f.grid = (n + f.cpb - 1) / f.cpb;
+            f.thr = (f.cpb * nb * f.split + 31) / 32 * 32;
+            return f;
+        };
+        const Shape fc = assemble_shape(nc), fs = assemble_shape(nbs);
+        k_adj_assemble<<<fc.grid, fc.thr, 0, s>>>(dm_, dp_, fc.cpb, fc.split, lam, eps, T_, Qbar, gcell, gtau);
+        k_adj_assemble_sides<<<fs.grid, fs.thr, 0, s>>>(dm_, dp_, fs.cpb, fs.split, eb_, ebb, dsum_, spec_src_, Qsbar,
+                                                        gtau, gbnd);
         CUDA_TRY(cudaGetLastError());
         gt.resize(nb);
         gc.resize(nc);
