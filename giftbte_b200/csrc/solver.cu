@@ -1612,19 +1612,21 @@ cudaError_t sweep_set_smem(int bytes) {
 //   E = sum_b S0 / C_bulk        (:2504)
 //   q = sum_b |v| S1             (:2515-2517)
 //   Th = kappa sum_{hr>0} lat S0 / C,  Q = sum_{hr>0} tau |v|^2 S2
-// (the two moments of the synthetic source). blockDim = cpb * nb. The band
-// sums of each cell are formed in shared memory in band order (no atomics),
-// so the moments are reproducible bit for bit.
+// (the two moments of the synthetic source). blockDim = cpb * nb / VE (rounded
+// up to a warp). The band sums of each cell are formed in shared memory in band
+// order (no atomics), so the moments are reproducible bit for bit.
+//
+// VE consecutive bands per thread: 2 in FP64 where the band count is even and
+// the blocks cover the SMs (16-byte accesses, and the ten weights that a warp
+// reads back from shared memory per direction serve twice the bands: 17,939
+// triangles x 40 x 64 0.254 -> 0.212 ms, 12,000 tetrahedra x 40 x 128 0.314 ->
+// 0.277 ms), 1 on smaller fields (288 triangles x 2 x 256, three blocks: 53 us,
+// 63 with half the warps) and in FP32 (2 there: 0.136 -> 0.149 ms on the
+// triangles).
 constexpr int kMomSlots = 12;
 constexpr int kWTab = 10;
 constexpr int kMomUnroll = 8;
 
-//
-// VE consecutive bands per thread: 2 in FP64 where the band count is even
-// (16-byte accesses, and the ten weights that a warp reads back from shared
-// memory per direction serve twice the bands: 17,939 triangles x 40 x 64
-// 0.254 -> 0.212 ms, 12,000 tetrahedra x 40 x 128 0.314 -> 0.277 ms), 1 in
-// FP32 (2 there: 0.136 -> 0.149 ms on the triangles, half the warps).
 template <typename S, int VE>
 __global__ void __launch_bounds__(256) k_moments(DMesh m, DPhys p, int cpb, S *__restrict__ eps,
                                                  const S *__restrict__ Dc, const double *__restrict__ Tb,
@@ -4377,7 +4379,7 @@ void Solver::launch_moments(S *eps, bool apply, int d0, int nbt, bool accumulate
                                                                     Tlat_, E_, q_, Tband_, Th_, Q_, apply ? 1 : 0, d0,
                                                                     nbt, accumulate ? 1 : 0);
     };
-    if (sizeof(S) == 8 && nb % 2 == 0)
+    if (sizeof(S) == 8 && nb % 2 == 0 && grid >= 148)
         go(std::integral_constant<int, 2>{});
     else
         go(std::integral_constant<int, 1>{});
