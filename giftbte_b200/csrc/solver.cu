@@ -2092,12 +2092,16 @@ __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int sp
     }
     if constexpr (MOM) {
         __syncthreads();
+        if (split > 1) {  // the shares of each (wall, band)
+            for (int t = threadIdx.x; t < rows * kWallSlots; t += blockDim.x)
+                for (int l = 1; l < split; l++) part[t] += part[(size_t)l * rows * kWallSlots + t];
+            __syncthreads();
+        }
         for (int t = threadIdx.x; t < cpb * kWallSlots; t += blockDim.x) {
             const int i = t / kWallSlots, j = t % kWallSlots, ww = blockIdx.x * cpb + i;
             if (ww >= nw) continue;
             double sum = 0;
-            for (int bb = 0; bb < nb; bb++)
-                for (int l = 0; l < split; l++) sum += part[((size_t)l * rows + i * nb + bb) * kWallSlots + j];
+            for (int bb = 0; bb < nb; bb++) sum += part[((size_t)i * nb + bb) * kWallSlots + j];
             const int s = wall_side[ww];
             if (j == 0) {
                 Ths[s] = (p.mat ? p.kap[p.mat[m.bs_cell[s]]] : p.kappa) * sum;
