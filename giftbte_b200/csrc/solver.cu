@@ -3707,16 +3707,18 @@ Error Solver::init(const FlatMesh &m, const Bands &b, const Angles &a, const std
             ws.push_back(sd);
         }
         n_walls_ = (int)ws.size();
-        cf_gw_ = up_i(gw);
         wall_side_ = up_i(ws);
-        wall_slot_ = up_i(slot);
+        if (face_path()) {
+            cf_gw_ = up_i(gw);
+            wall_slot_ = up_i(slot);
+        }
     }
     if (!ok) return {-6, "device allocation or upload failed"};
     Error e = alloc_all();
     if (e.code) return e;
-    if (mesh.dim == 2)
+    if (face_mask_ && mesh.dim == 2)
         k_face_mask<2><<<grid_for((size_t)nd * mesh.nc), kThreads, 0, s>>>(dm_, dp_, face_mask_);
-    else
+    else if (face_mask_)
         k_face_mask<3><<<grid_for((size_t)nd * mesh.nc), kThreads, 0, s>>>(dm_, dp_, face_mask_);
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(s));
@@ -3783,10 +3785,14 @@ Error Solver::alloc_all() {
     // directions when they fit in 90% of the free device memory, else
     // batches of directions (the intensities, records and schedules stay whole)
     {
-        // (the gradient buffer also holds the face values of the face-value
-        // path, one row per face; wall_grad_ its gradients at wall faces)
-        const size_t grows = std::max(nc * mesh.dim, (size_t)mesh.nf());
-        const size_t per_dir = nb * S * (grows + 2 * nc + (size_t)n_wall_slots_ * mesh.dim);
+        // a handle that can take the face-value path: the gradient buffer also
+        // holds the face values, one row per face; wall_grad_ the gradients at
+        // wall faces. (Its mask is whole: allocated before the room is measured.)
+        const bool faces = face_path();
+        if (faces) face_mask_ = (unsigned char *)A(nd * nc);
+        const size_t grows = faces ? std::max(nc * mesh.dim, (size_t)mesh.nf()) : nc * mesh.dim;
+        const size_t wrows = faces ? (size_t)n_wall_slots_ * mesh.dim : 0;
+        const size_t per_dir = nb * S * (grows + 2 * nc + wrows);
         size_t fr = 0, tot = 0;
         CUDA_TRY(cudaMemGetInfo(&fr, &tot));
         const size_t room = fr > (size_t)512 << 20 ? (size_t)((fr - ((size_t)512 << 20)) * 0.9) : 0;
@@ -3794,13 +3800,13 @@ Error Solver::alloc_all() {
         if (cfg.direction_batch > 0) ndb_ = std::min(ndb_, cfg.direction_batch);
         if (ndb_ < 1) return {-6, "device memory too small for one direction's gradient/residual buffers"};
         grad_ = A((size_t)ndb_ * grows * nb * S);
-        wall_grad_ = A(std::max<size_t>(1, (size_t)ndb_ * n_wall_slots_ * mesh.dim * nb) * S);
-        face_mask_ = (unsigned char *)A(nd * nc);
+        if (faces) wall_grad_ = A((size_t)ndb_ * wrows * nb * S);
         res_ = A((size_t)ndb_ * nc * nb * S);
         corr_ = A((size_t)ndb_ * nc * nb * S);
     }
-    for (void *pp : {grad_, res_, corr_, wall_grad_, (void *)face_mask_, (void *)Tbase_, (void *)Bflux_, (void *)eb_, (void *)cg_scal_})
-        if (!pp)
+    const bool faces_missing = face_path() && (!wall_grad_ || !face_mask_);
+    for (void *pp : {grad_, res_, corr_, (void *)Tbase_, (void *)Bflux_, (void *)eb_, (void *)cg_scal_})
+        if (!pp || faces_missing)
             return {-6, "device allocation failed (" + std::to_string(ne * S * (3 + mesh.dim) / 1048576) +
                             " MiB of band state)"};
     if (cudaMallocHost((void **)&h_pinned_, 64 * sizeof(double)) != cudaSuccess) return {-6, "pinned allocation failed"};
