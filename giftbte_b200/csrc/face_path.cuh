@@ -61,27 +61,37 @@ __global__ void __launch_bounds__(256) k_face_mask(DMesh m, DPhys p, unsigned ch
     }
 }
 
-// loads from a shared-memory address (32-bit)
+// loads from a shared-memory address (32-bit); what they read was written by
+// ordinary stores and by cp.async, hence the clobber
 __device__ __forceinline__ void lds(unsigned a, float (&v)[4]) {
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(a));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                 : "r"(a)
+                 : "memory");
 }
 __device__ __forceinline__ void lds(unsigned a, double (&v)[2]) {
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a));
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void lds(unsigned a, FaceW<float, 2> &t) {
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=r"(t.at) : "r"(a));
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=r"(t.at)
+                 : "r"(a)
+                 : "memory");
 }
 __device__ __forceinline__ void lds(unsigned a, FaceW<float, 3> &t) {
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=r"(t.at) : "r"(a));
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=r"(t.at)
+                 : "r"(a)
+                 : "memory");
 }
 __device__ __forceinline__ void lds(unsigned a, FaceW<double, 2> &t) {
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t.x), "=d"(t.y) : "r"(a));
-    asm volatile("ld.shared.b32 %0, [%1+16];" : "=r"(t.at) : "r"(a));
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t.x), "=d"(t.y) : "r"(a) : "memory");
+    asm volatile("ld.shared.b32 %0, [%1+16];" : "=r"(t.at) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void lds(unsigned a, FaceW<double, 3> &t) {
     double w;
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t.x), "=d"(t.y) : "r"(a));
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2+16];" : "=d"(t.z), "=d"(w) : "r"(a));
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(t.x), "=d"(t.y) : "r"(a) : "memory");
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2+16];" : "=d"(t.z), "=d"(w) : "r"(a) : "memory");
     t.at = __double2loint(w);
 }
 
