@@ -4086,7 +4086,6 @@ bool Solver::face_path() const {
 template <typename S, int DIM>
 Error Solver::face_shape() {
     if (fshape_built_) return {0, ""};
-    fshape_built_ = true;
     cudaStream_t s = cfg.stream;
     // The widest block of which two fit on an SM (227 KB, 1 KB of it per block
     // for the system), else the widest that fits at all: its shared memory is
@@ -4120,16 +4119,22 @@ Error Solver::face_shape() {
             if (ce.code) return ce;
         }
         bool ok = true;
+        const size_t held = allocs_.size();
         f.tile.B = t.B, f.tile.nblk = t.nblk, f.tile.umax = t.umax, f.tile.qmax = t.qmax;
         f.tile.ptr = upload(this, allocs_, t.ptr, s, ok);
         f.tile.cells = upload(this, allocs_, t.cells, s, ok);
         f.tile.loc = upload(this, allocs_, t.loc, s, ok);
-        if (!ok) return {-6, "device allocation failed (gradient tiles)"};
         CUDA_TRY(cudaStreamSynchronize(s));
+        if (!ok) {
+            for (; allocs_.size() > held; allocs_.pop_back()) cudaFree(allocs_.back());
+            cudaGetLastError();  // reported here, not by the next call's check
+            return {-6, "device allocation failed (gradient tiles)"};
+        }
         CUDA_TRY(cudaFuncSetAttribute(k_grad_face<S, DIM, kFaceW<S, DIM>, kFaceNP<DIM>>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         fshape_ = f;
     }
+    fshape_built_ = true;  // only now: what failed above (memory) is tried again, not taken as "none fits"
     return {0, ""};
 }
 
