@@ -2470,7 +2470,8 @@ __device__ __forceinline__ double warp_allsum(double v) {
 // it has this CTA's sums, which follow its halo reads. The sums alternate
 // between two buffers and two barriers: a fast CTA can be one exchange ahead
 // of a slow one, never two. Every wait gives up after kCgTries polls; the CTA
-// then leaves the loop as a whole. The number of remote stores matters more
+// then leaves the loop as a whole and stays until what may still be on its way
+// to it has arrived. The number of remote stores matters more
 // than the kind of barrier: the 3 x 16 aggregate sums of 16 CTAs as 8-byte
 // stores took 2,400 clocks an exchange, 16 bytes at a time with those of r
 // and s sent ahead of the product A u about 900 (cluster barrier 480, one
@@ -2798,8 +2799,14 @@ __global__ void __launch_bounds__(kCgThreads, 1)
     }
     // every CTA has left the loop, its last sums in place, before a buffer is
     // written again
-    if (lost) *cl.map_shared_rank(gone, 0) = 1;
+    const bool gave_up = __syncthreads_or(lost);
+    if (gave_up && tid == 0) *cl.map_shared_rank(gone, 0) = 1;
     cl.sync();
+    // A CTA that waited for all it was sent has nothing under way to it. One
+    // that gave up may: no CTA sends any more, so it gives the stores that are
+    // still in flight a millisecond before its shared memory goes.
+    if (gave_up)
+        for (int k = 0; k < 64; k++) __nanosleep(16384);
     double sq = 0;
     for (int i = tid; i < nr; i += bd) {
         const int o = perm[base + i];
