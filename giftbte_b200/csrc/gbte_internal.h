@@ -204,6 +204,20 @@ Error make_angles(int method, int ntheta, int nphi, int material_dim, Angles &ou
 // an explicit direction set: unit vectors [n * 3], weights summing to the solid angle
 Error explicit_angles(int n, const double *xyz, const double *weight, double solid, Angles &out);
 Error build_flat_mesh(const RawMesh &raw, const BCs &bcs, const Bands &bands, FlatMesh &out);
+
+// The walls as the wall kernels walk them. Every cell face on a boundary has a
+// slot (cf_slot; -1 on interior faces), where the face-value path keeps its
+// gradient. side lists every boundary side that has a cell, first the one that
+// each slot's face refers to, in slot order, then the sides that name a face
+// again (a boundary element given twice, or a tag in two rows of the boundary
+// table), which periodic partners and node values may refer to; slot is the
+// slot of each listed side's face.
+struct WallTable {
+    int nslots = 0;
+    std::vector<int> cf_slot;     // [cell-face slots]
+    std::vector<int> side, slot;  // [walls]
+};
+void build_wall_table(const FlatMesh &m, WallTable &out);
 void build_schedule(const FlatMesh &m, const Angles &a, Schedule &out, int nthreads);
 // min_ring: the smallest ring (rounded up to a power of two and to the
 // widest level); far_cap: most far slots allowed, 0 disables them. The
@@ -260,5 +274,10 @@ bool index_checks_enabled();
 Error check_indices(const FlatMesh &m, int nb, const Schedule &s, int nd, const SweepPlan &sp, long long &checked);
 // the same for the shared-memory tiles (either may be null)
 Error check_tiles(const FlatMesh &m, const GradTiles *g, const FaceTiles *f, long long &checked);
+// for the wall table: slots and sides name each other's faces, and every side
+// with a cell is listed once
+Error check_walls(const FlatMesh &m, const WallTable &w, long long &checked);
+// and for the columns of a macro system in ELL form: count entries below bound
+Error check_columns(const char *name, const std::vector<int> &col, size_t count, int bound, long long &checked);
 
 }  // namespace gbte

@@ -563,6 +563,24 @@ Error build_flat_mesh(const RawMesh &raw, const BCs &bcs, const Bands &bands, Fl
     return {0, ""};
 }
 
+void build_wall_table(const FlatMesh &m, WallTable &out) {
+    out = WallTable();
+    out.cf_slot.assign(m.ncf(), -1);
+    for (int k = 0; k < m.ncf(); k++)
+        if (m.cf_bound[k] >= 0) {
+            out.cf_slot[k] = (int)out.side.size();
+            out.slot.push_back(out.cf_slot[k]);
+            out.side.push_back(m.cf_bside[k]);
+        }
+    out.nslots = (int)out.side.size();
+    for (int s = 0; s < m.nbs(); s++) {
+        const int k = m.bs_cell[s] < 0 ? -1 : m.bs_cf[s];
+        if (k < 0 || m.cf_bside[k] == s) continue;
+        out.slot.push_back(out.cf_slot[k]);
+        out.side.push_back(s);
+    }
+}
+
 // Upwind level schedule per direction (Kahn's algorithm). Cell c depends on
 // interior neighbour o across face k when s_d . n_k < 0. Faces that close a
 // cycle (possible on distorted 3D tetrahedra) are lagged: the sweep treats
@@ -1266,6 +1284,40 @@ Error check_tiles(const FlatMesh &m, const GradTiles *g, const FaceTiles *f, lon
             }
         }
     }
+    checked = c.n;
+    if (!c.ok()) return {-7, "index check: " + c.err};
+    return {0, ""};
+}
+
+Error check_walls(const FlatMesh &m, const WallTable &w, long long &checked) {
+    IndexCheck c;
+    const int nbs = m.nbs();
+    c.size("wall cf_slot", w.cf_slot.size(), (size_t)m.ncf());
+    c.size("wall slot", w.slot.size(), w.side.size());
+    c.range("wall cf_slot", w.cf_slot, -1, w.nslots);
+    c.range("wall side", w.side, 0, nbs);
+    c.range("wall slot", w.slot, 0, w.nslots);
+    for (int k = 0; k < m.ncf() && c.ok(); k++)
+        if ((w.cf_slot[k] >= 0) != (m.cf_bound[k] >= 0))
+            c.fail("wall cf_slot[" + std::to_string(k) + "]: a slot on an interior face, or none on a wall");
+    std::vector<char> seen(nbs, 0);
+    for (size_t i = 0; i < w.side.size() && c.ok(); i++) {
+        const int s = w.side[i];
+        if (m.bs_cell[s] < 0 || seen[s]++) c.fail("wall side[" + std::to_string(i) + "]: without a cell, or listed twice");
+        if (c.ok() && w.cf_slot[m.bs_cf[s]] != w.slot[i])
+            c.fail("wall slot[" + std::to_string(i) + "] is another face's");
+    }
+    for (int s = 0; s < nbs && c.ok(); s++)
+        if (m.bs_cell[s] >= 0 && !seen[s]) c.fail("wall side " + std::to_string(s) + " is not listed");
+    checked = c.n;
+    if (!c.ok()) return {-7, "index check: " + c.err};
+    return {0, ""};
+}
+
+Error check_columns(const char *name, const std::vector<int> &col, size_t count, int bound, long long &checked) {
+    IndexCheck c;
+    c.size(name, col.size(), count);
+    c.range(name, col, 0, bound);
     checked = c.n;
     if (!c.ok()) return {-7, "index check: " + c.err};
     return {0, ""};

@@ -3470,31 +3470,20 @@ Error Solver::init(const FlatMesh &m, const Bands &b, const Angles &a, const std
         bTF_ = up_d(bT);
         bF_dir_ = up_i(dir);
     }
-    // wall slot of every wall face of a cell (-1 on interior faces), and the
-    // wall sides: the one each slot's face refers to, in slot order, then the
-    // sides that name a face again (a boundary element given twice, or a tag
-    // in two rows of the boundary table), which periodic partners and node
-    // values may refer to
     {
-        std::vector<int> gw(mesh.ncf(), -1), ws, slot;
-        for (int k = 0; k < mesh.ncf(); k++)
-            if (mesh.cf_bound[k] >= 0) {
-                gw[k] = (int)ws.size();
-                slot.push_back(gw[k]);
-                ws.push_back(mesh.cf_bside[k]);
-            }
-        n_wall_slots_ = (int)ws.size();
-        for (int sd = 0; sd < mesh.nbs(); sd++) {
-            const int k = mesh.bs_cell[sd] < 0 ? -1 : mesh.bs_cf[sd];
-            if (k < 0 || mesh.cf_bside[k] == sd) continue;
-            slot.push_back(gw[k]);
-            ws.push_back(sd);
+        WallTable wt;
+        build_wall_table(mesh, wt);
+        if (index_checks_enabled()) {
+            long long checked = 0;
+            Error ce = check_walls(mesh, wt, checked);
+            if (ce.code) return ce;
         }
-        n_walls_ = (int)ws.size();
-        wall_side_ = up_i(ws);
+        n_wall_slots_ = wt.nslots;
+        n_walls_ = (int)wt.side.size();
+        wall_side_ = up_i(wt.side);
         if (face_path()) {
-            cf_gw_ = up_i(gw);
-            wall_slot_ = up_i(slot);
+            cf_gw_ = up_i(wt.cf_slot);
+            wall_slot_ = up_i(wt.slot);
         }
     }
     if (!ok) return {-6, "device allocation or upload failed"};
@@ -3929,6 +3918,11 @@ Error Solver::cg_plan(const std::vector<int> &ptr, const std::vector<int> &idx, 
             sdst[(size_t)k * smax + e] = sends[k][e].second;
         }
     }
+    if (index_checks_enabled()) {
+        long long checked = 0;
+        Error ce = check_columns("cluster columns", ec, std::max<size_t>(ell, 1), nrmax + hmax, checked);
+        if (ce.code) return ce;
+    }
     // coarse level: Ac = R A R^T over the aggregates, inverted on the host
     bool coarse = true;
     for (int g = 0; g < NA && coarse; g++) coarse = abounds[g + 1] - abounds[g] >= 4;
@@ -4054,6 +4048,11 @@ Error Solver::ell_plan(const std::vector<int> &ptr, const std::vector<int> &idx,
             col[(size_t)e * n + i] = q < ptr[i + 1] ? idx[q] : i;
             if (q < ptr[i + 1]) v[(size_t)e * n + i] = val[q];
         }
+    }
+    if (index_checks_enabled()) {
+        long long checked = 0;
+        Error ce = check_columns("macro columns", col, (size_t)kEll * n, n, checked);
+        if (ce.code) return ce;
     }
     bool ok = true;
     pl.gcol = upload(this, allocs_, col, cfg.stream, ok);
