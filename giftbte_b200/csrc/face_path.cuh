@@ -36,6 +36,9 @@ template <typename S, int DIM> struct FaceW;
 template <int DIM> struct alignas(16) FaceW<float, DIM> { float x, y, z; int at; };
 template <> struct alignas(16) FaceW<double, 3> { double x, y, z; int at, pad; };
 template <> struct alignas(16) FaceW<double, 2> { double x, y; int at, pad[3]; };
+static_assert(sizeof(FaceW<float, 2>) == face_entry_bytes(4) && sizeof(FaceW<float, 3>) == face_entry_bytes(4) &&
+                  sizeof(FaceW<double, 2>) == face_entry_bytes(8) && sizeof(FaceW<double, 3>) == face_entry_bytes(8),
+              "the host sizes the tiles");
 
 // Which side of every face its upwind value comes from: bit j of
 // mask[d][c] is set when cell c writes the value of its face j in direction

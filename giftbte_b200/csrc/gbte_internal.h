@@ -240,6 +240,20 @@ struct GradTiles {
 };
 Error build_grad_tiles(const FlatMesh &m, int B, GradTiles &out);
 
+// Tiles of the face-value gradient. A cell has face_lanes threads, each with
+// face_pieces 16-byte pieces of a band row (size: bytes of a stored
+// intensity): 4 lanes of 2 pieces in 2D FP32 and 8 of 2 in 2D FP64 (one stencil
+// entry serves two row loads), 8 of 1 in 3D (a wider slab would leave one CTA
+// per SM).
+constexpr int face_lanes(int dim, size_t size) { return dim == 2 && size == 4 ? 4 : 8; }
+constexpr int face_pieces(int dim) { return dim == 2 ? 2 : 1; }
+constexpr size_t face_entry_bytes(size_t size) { return size == 4 ? 16 : 32; }  // a staged stencil entry or face
+// the shared memory of a CTA on the blocks of t
+size_t face_tile_smem(const GradTiles &t, int dim, size_t size);
+// The widest blocks of which two fit on an SM, else the widest that fit at all
+// (out.B = 0: none).
+Error build_face_path_tiles(const FlatMesh &m, size_t size, GradTiles &out);
+
 // Shared memory of a CTA of the face-value residual: the band constants of
 // every material and the coefficients of its cells and kResDirs directions.
 // nb * size is a multiple of 16 (size: bytes of a stored intensity).

@@ -1045,6 +1045,33 @@ Error build_grad_tiles(const FlatMesh &m, int B, GradTiles &out) {
     return {0, ""};
 }
 
+size_t face_tile_smem(const GradTiles &t, int dim, size_t size) {
+    return ((size_t)t.qmax + 4 * t.B) * face_entry_bytes(size) +
+           (size_t)t.umax * (face_lanes(dim, size) * face_pieces(dim) * 16 + sizeof(int));
+}
+
+// Cells per block: 32 in 2D and in the 3D FP32 form, 24 in the 3D FP64 form
+// (its stencil entries are 32 bytes), fewer where the tiles of two blocks do
+// not fit on an SM (227 KB, 1 KB of it per block for the system): a block's
+// shared memory is the mesh's largest union, so a width that pairs on one mesh
+// may not on the next. 1.92 million tetrahedra x 40 bands x 64 directions
+// (FP32): 32 cells, one block per SM 126.9 ms; 28 cells, two 100.6; 24 104.7;
+// 16 126.4.
+Error build_face_path_tiles(const FlatMesh &m, size_t size, GradTiles &out) {
+    out = GradTiles();
+    const int best = m.dim == 3 && size == 8 ? 24 : 32, step = 32 / face_lanes(m.dim, size);
+    int width = 0;
+    for (int B = best; B >= (out.B ? 16 : 8) && width == 0; B -= B > 16 ? step : 8) {
+        GradTiles t;
+        if (build_grad_tiles(m, B, t).code) continue;
+        const size_t smem = face_tile_smem(t, m.dim, size);
+        const bool pairs = smem <= 227 * 1024 / 2 - 1024;
+        if (pairs || (B <= 16 && out.B == 0 && smem <= 220 * 1024)) width = B;
+        if (width || (out.B == 0 && smem <= 220 * 1024)) out = std::move(t);
+    }
+    return {0, ""};
+}
+
 Error build_face_tiles(const FlatMesh &m, int B, FaceTiles &out) {
     out = FaceTiles();
     if (B < 1 || B > 1024) return {-1, "residual tile size out of range"};

@@ -4062,12 +4062,6 @@ Error Solver::ell_plan(const std::vector<int> &ptr, const std::vector<int> &idx,
     return {0, ""};
 }
 
-// lanes per cell and pieces per lane of the face-value gradient
-template <typename S, int DIM>
-constexpr int kFaceW = DIM == 2 && sizeof(S) == 4 ? 4 : 8;
-template <int DIM>
-constexpr int kFaceNP = DIM == 2 ? 2 : 1;
-
 // The face-value path serves the second-order scheme without the limiter
 // when a band row is a whole number of 16-byte pieces; a launch shape fixed
 // by the caller (options.gradient_dirs, residual_form) keeps the
@@ -4084,41 +4078,17 @@ bool Solver::face_path() const {
            (size_t)std::max(mesh.nc, mesh.nf()) * bands.nb < ((size_t)1 << 31);
 }
 
-// Cells per block: 32 in 2D and in the 3D FP32 form, 24 in the 3D FP64 form
-// (its stencil entries are 32 bytes), fewer where the tiles of two blocks do
-// not fit on an SM. Pieces and lanes per cell: 4 lanes of
-// 2 pieces in 2D FP32 and 8 of 2 in 2D FP64 (one stencil entry serves two
-// row loads), 8 of 1 in 3D (a wider slab would leave one CTA per SM).
 template <typename S, int DIM>
 Error Solver::face_shape() {
     if (fshape_built_) return {0, ""};
     cudaStream_t s = cfg.stream;
-    // The widest block of which two fit on an SM (227 KB, 1 KB of it per block
-    // for the system), else the widest that fits at all: its shared memory is
-    // the mesh's largest union, so a width that pairs on one mesh may not on
-    // the next. 1.92 million tetrahedra x 40 bands x 64 directions (FP32): 32
-    // cells, one block per SM 126.9 ms; 28 cells, two 100.6; 24 104.7; 16 126.4.
-    constexpr int W = kFaceW<S, DIM>, best = DIM == 3 && sizeof(S) == 8 ? 24 : 32, step = 32 / W;
-    auto smem_of = [&](const GradTiles &t, int B) {
-        return ((size_t)t.qmax + 4 * B) * sizeof(FaceW<S, DIM>) +
-               (size_t)t.umax * (W * kFaceNP<DIM> * 16 + sizeof(int));
-    };
-    int width = 0;
-    GradTiles pick;
-    for (int B = best; B >= (pick.B ? 16 : 8) && width == 0; B -= B > 16 ? step : 8) {
-        GradTiles t;
-        if (build_grad_tiles(mesh, B, t).code) continue;
-        const size_t smem = smem_of(t, B);
-        const bool pairs = smem <= 227 * 1024 / 2 - 1024;
-        if (pairs || (B <= 16 && pick.B == 0 && smem <= 220 * 1024)) width = B;
-        if (width || (pick.B == 0 && smem <= 220 * 1024)) pick = std::move(t);
-    }
-    if (pick.B > 0) {
-        const GradTiles &t = pick;
-        const int B = t.B;
+    GradTiles t;
+    Error te = build_face_path_tiles(mesh, sizeof(S), t);
+    if (te.code) return te;
+    if (t.B > 0) {
         FaceShape f;
-        f.threads = B * W;
-        f.smem = smem_of(t, B);
+        f.threads = t.B * face_lanes(DIM, sizeof(S));
+        f.smem = face_tile_smem(t, DIM, sizeof(S));
         if (index_checks_enabled()) {
             long long checked = 0;
             Error ce = check_tiles(mesh, &t, nullptr, checked);
@@ -4136,7 +4106,7 @@ Error Solver::face_shape() {
             cudaGetLastError();  // reported here, not by the next call's check
             return {-6, "device allocation failed (gradient tiles)"};
         }
-        CUDA_TRY(cudaFuncSetAttribute(k_grad_face<S, DIM, kFaceW<S, DIM>, kFaceNP<DIM>>,
+        CUDA_TRY(cudaFuncSetAttribute(k_grad_face<S, DIM, face_lanes(DIM, sizeof(S)), face_pieces(DIM)>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         fshape_ = f;
     }
@@ -4146,7 +4116,7 @@ Error Solver::face_shape() {
 
 template <typename S, int DIM>
 cudaError_t Solver::launch_grad_face(const S *eps, int d0, int nbt) {
-    constexpr int W = kFaceW<S, DIM>, NP = kFaceNP<DIM>, SW = W * NP;
+    constexpr int W = face_lanes(DIM, sizeof(S)), NP = face_pieces(DIM), SW = W * NP;
     const FaceShape &f = fshape_;
     const int nb = bands.nb, ppd = nb / kPieceBands<S>;
     const int slabs = (nbt * ppd + SW - 1) / SW;
