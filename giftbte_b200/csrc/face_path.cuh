@@ -418,25 +418,28 @@ __global__ void __launch_bounds__(256, 3) k_resid_face(DMesh m, DPhys p, int cpb
 
 // The explicit time step (FP64, base 0) from the face values, in place:
 // e <- e (1 - dt/tau) - dt (sum_f A/V (v.n) x_f - C Told/tau). A thread keeps
-// a 16-byte piece of a cell's bands over kResDirs directions, as k_resid_face
-// does; only the thread that writes a value reads it, so the new field needs
-// no second array and no copy back. Bound by the face rows it streams.
+// a 16-byte piece of a cell's bands over `dirs` directions (kResDirs, as
+// k_resid_face does, or fewer where that leaves SMs without a block); only the
+// thread that writes a value reads it, so the new field needs no second array
+// and no copy back. Bound by the face rows it streams.
 // 4,608 triangles x 20 bands x 32 directions (FP64): 27 us, and a whole step
 // 287 -> 159 us against gradient arrays, a thread per value and a copy back.
+// 288 triangles x 2 bands x 256 directions: 27.6 us with eight directions each,
+// 16.6 us with four.
 template <int DIM>
-__global__ void __launch_bounds__(256, 3) k_tr_step_face(DMesh m, DPhys p, int cpb, double *eps,
+__global__ void __launch_bounds__(256, 3) k_tr_step_face(DMesh m, DPhys p, int cpb, int dirs, double *eps,
                                                          const double *__restrict__ F,
                                                          const unsigned char *__restrict__ mask,
                                                          const double *__restrict__ Told,
                                                          const double *__restrict__ eb, double dt, int d0, int ndb) {
     constexpr int VE = kPieceBands<double>;
     extern __shared__ __align__(16) unsigned char rfm[];
-    double *coef = reinterpret_cast<double *>(rfm);  // [kResDirs][cpb][4]
+    double *coef = reinterpret_cast<double *>(rfm);  // [dirs][cpb][4]
     const int nb = p.nb, nc = m.nc, nf = m.nf, ppd = nb / VE;
     const int cb = blockIdx.x * cpb, ncell = min(cpb, nc - cb);
-    const int da = blockIdx.y * kResDirs, nd = min(kResDirs, ndb - da);
+    const int da = blockIdx.y * dirs, nd = min(dirs, ndb - da);
     const int tid = threadIdx.x;
-    for (int t = tid; t < kResDirs * cpb * 4; t += blockDim.x) {
+    for (int t = tid; t < dirs * cpb * 4; t += blockDim.x) {
         const int j = t & 3, ci = (t >> 2) % cpb, dd = (t >> 2) / cpb;
         double a = 0;
         if (ci < ncell && dd < nd) {

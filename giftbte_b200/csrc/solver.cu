@@ -5174,9 +5174,11 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
             if (faces) {
                 CUDA_TRY((launch_grad_face<double, DIM>(eps, d0, nbt)));
                 const int ppd = nb / kPieceBands<double>, cpb = resid_face_cells(nb, sizeof(double));
-                const dim3 grid((nc + cpb - 1) / cpb, (nbt + kResDirs - 1) / kResDirs);
-                k_tr_step_face<DIM><<<grid, (cpb * ppd + 31) / 32 * 32, (size_t)kResDirs * cpb * 4 * 8, s>>>(
-                    dm_, dp_, cpb, eps, g, face_mask_, T_, eb_, dt, d0, nbt);
+                int dirs = kResDirs;
+                while (dirs > 1 && (nc + cpb - 1) / cpb * ((nbt + dirs - 1) / dirs) < 148) dirs /= 2;
+                const dim3 grid((nc + cpb - 1) / cpb, (nbt + dirs - 1) / dirs);
+                k_tr_step_face<DIM><<<grid, (cpb * ppd + 31) / 32 * 32, (size_t)dirs * cpb * 4 * 8, s>>>(
+                    dm_, dp_, cpb, dirs, eps, g, face_mask_, T_, eb_, dt, d0, nbt);
             } else {
                 k_gradient<double, DIM><<<grid_for(nbe), kThreads, 0, s>>>(dm_, dp_, w, eps, g, d0, nbt);
                 k_tr_step<DIM><<<grid_for(nbe), kThreads, 0, s>>>(dm_, dp_, ev, T_, eb_, dt, R, d0, nbt);
