@@ -102,7 +102,7 @@ dim3 wall_grid(size_t items, int nd) {
 
 // The passes that set up the stored deviations and their base. Each owns what
 // does not depend on the direction (a cell's band, a cell's faces) and walks
-// `per` directions of its share, so the cell's index arithmetic, constants
+// kDirShare directions, so the cell's index arithmetic, constants
 // and FP64 face geometry are formed once for all of them; bound by the HBM
 // traffic of the band state. 48,000 tetrahedra x 40 bands x 128 directions
 // (FP32), against a thread per value: init 0.64 -> 0.15 ms, rebase 0.77 ->

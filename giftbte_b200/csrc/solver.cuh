@@ -88,6 +88,9 @@ struct SolverConfig {
     bool own_stream = false;
 };
 
+// Ids of the per-kernel times (gbte_kernel_name). K_GATHER is the whole wall
+// kernel: moments, refresh and wall temperatures; K_SIDE_MOMENTS and K_MACRO_BC
+// keep their places for callers that hold the ids, without launches of their own.
 enum KernelId {
     K_GRADIENT = 0, K_RESIDUAL, K_SWEEP, K_BOUND_OUT, K_MOMENTS, K_SIDE_MOMENTS, K_NODE_INTERP, K_REMACRO,
     K_GATHER, K_MACRO_BC, K_TINTERP, K_MACRO_RHS, K_PCG, K_REDUCE, K_COPY, K_INIT, K_NUM
