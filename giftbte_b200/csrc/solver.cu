@@ -1622,7 +1622,9 @@ cudaError_t sweep_set_smem(int bytes) {
 // triangles x 40 x 64 0.254 -> 0.212 ms, 12,000 tetrahedra x 40 x 128 0.314 ->
 // 0.277 ms), 1 on smaller fields (288 triangles x 2 x 256, three blocks: 53 us,
 // 63 with half the warps) and in FP32 (2 there: 0.136 -> 0.149 ms on the
-// triangles).
+// triangles). The FP32 form is at 64 registers, four blocks per SM: the
+// constants of the end are formed at the start for it (at 72, with three
+// blocks, 147 us on the triangles instead of 135).
 constexpr int kMomSlots = 12;
 constexpr int kWTab = 10;
 constexpr int kMomUnroll = 8;
@@ -1637,18 +1639,19 @@ __global__ void __launch_bounds__(256) k_moments(DMesh m, DPhys p, int cpb, S *_
                                                  int accumulate) {
     extern __shared__ double sm_dyn[];
     const int nb = p.nb, nc = m.nc, tpc = nb / VE;  // threads per cell
-    double *wt = sm_dyn;                             // [ndb][kWTab]
+    double *wt = sm_dyn;                             // [nd][kWTab]
     double *part = sm_dyn + (size_t)p.nd * kWTab;    // [cpb][nb][kMomSlots]
-    for (int i = threadIdx.x; i < ndb * kWTab; i += blockDim.x) wt[i] = wtab[(size_t)d0 * kWTab + i];
+    for (int i = threadIdx.x; i < p.nd * kWTab; i += blockDim.x) wt[i] = wtab[i];
     __syncthreads();
-    const int lc = threadIdx.x / tpc, b0 = (threadIdx.x - lc * tpc) * VE;
+    const int lc = threadIdx.x / tpc, b0 = threadIdx.x % tpc * VE;
     const int c = blockIdx.x * cpb + lc;
     if (lc < cpb && c < nc) {
         const int mo = mat_off(p, c);
-        double base[VE], a[VE][kWTab];
+        double *mine0 = part + VE * threadIdx.x * kMomSlots;  // [lc][b0]
+        double base[VE], cb[VE], a[VE][kWTab];
 #pragma unroll
         for (int v = 0; v < VE; v++) {
-            base[v] = p.C[mo + b0 + v] * Tb[c];
+            cb[v] = p.C[mo + b0 + v], base[v] = cb[v] * Tb[c];
 #pragma unroll
             for (int i = 0; i < kWTab; i++) a[v][i] = 0;
         }
@@ -1670,14 +1673,14 @@ __global__ void __launch_bounds__(256) k_moments(DMesh m, DPhys p, int cpb, S *_
 #pragma unroll
             for (int u = 0; u < kMomUnroll; u++) {
                 if (d + u >= ndb) break;
+                S en[VE];
                 double e[VE];
 #pragma unroll
-                for (int v = 0; v < VE; v++) {
-                    ev[u][v] += dv[u][v];
-                    e[v] = base[v] + (double)ev[u][v];
-                }
-                if (apply) vst<S, VE>(e0 + (size_t)(d + u) * stride, ev[u]);
-                const double *w = wt + kWTab * (d + u);
+                for (int v = 0; v < VE; v++) en[v] = ev[u][v] + dv[u][v];
+                if (apply) vst<S, VE>(e0 + (size_t)(d + u) * stride, en);
+#pragma unroll
+                for (int v = 0; v < VE; v++) e[v] = base[v] + (double)en[v];
+                const double *w = wt + kWTab * (d0 + d + u);
 #pragma unroll
                 for (int i = 0; i < kWTab; i++)
 #pragma unroll
@@ -1687,8 +1690,8 @@ __global__ void __launch_bounds__(256) k_moments(DMesh m, DPhys p, int cpb, S *_
 #pragma unroll
         for (int v = 0; v < VE; v++) {
             const int b = b0 + v;
-            double *mine = part + ((size_t)lc * nb + b) * kMomSlots;
-            const double Cb = p.C[mo + b];
+            double *mine = mine0 + v * kMomSlots;  // = lc * nb + b
+            const double Cb = cb[v];
             if (accumulate)
                 Tband[(size_t)b * nc + c] += a[v][0] / Cb;
             else
@@ -4147,10 +4150,9 @@ void Solver::launch_moments(S *eps, bool apply, int d0, int nbt, bool accumulate
                                                                     Tlat_, E_, q_, Tband_, Th_, Q_, apply ? 1 : 0, d0,
                                                                     nbt, accumulate ? 1 : 0);
     };
-    if (sizeof(S) == 8 && nb % 2 == 0 && grid >= 148)
-        go(std::integral_constant<int, 2>{});
-    else
-        go(std::integral_constant<int, 1>{});
+    if constexpr (sizeof(S) == 8)
+        if (nb % 2 == 0 && grid >= 148) return go(std::integral_constant<int, 2>{});
+    go(std::integral_constant<int, 1>{});
 }
 
 // the wall kernel, with or without the moments (outside the solve's stages
@@ -4334,7 +4336,8 @@ Error Solver::solve_t(SolveStats &st) {
     if (nb > 256) return {-8, "more than 256 bands are not supported"};
     if (msmem > 48 * 1024) {
         CUDA_TRY((cudaFuncSetAttribute(k_moments<S, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
-        CUDA_TRY((cudaFuncSetAttribute(k_moments<S, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
+        if constexpr (sizeof(S) == 8)
+            CUDA_TRY((cudaFuncSetAttribute(k_moments<S, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     }
     if (msmem > 40 * 1024)
         CUDA_TRY(cudaFuncSetAttribute(k_walls<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
