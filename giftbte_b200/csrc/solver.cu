@@ -1617,12 +1617,14 @@ cudaError_t sweep_set_smem(int bytes) {
 // order (no atomics), so the moments are reproducible bit for bit.
 //
 // VE consecutive bands per thread: 2 in FP64 where the band count is even and
-// the blocks cover the SMs (16-byte accesses, and the ten weights that a warp
-// reads back from shared memory per direction serve twice the bands: 17,939
-// triangles x 40 x 64 0.254 -> 0.212 ms, 12,000 tetrahedra x 40 x 128 0.314 ->
-// 0.277 ms), 1 on smaller fields (288 triangles x 2 x 256, three blocks: 53 us,
-// 63 with half the warps) and in FP32 (2 there: 0.136 -> 0.149 ms on the
-// triangles). The FP32 form is at 64 registers, four blocks per SM: the
+// the launch then takes fewer waves, three blocks of half the threads on an SM
+// against two. A block itself is 4% to 16% slower for it, although its accesses
+// have 16 bytes and the ten weights that a warp reads back from shared memory
+// per direction serve twice the bands. 64 directions, one band and two, us: 281
+// blocks (one wave each) 24.3 and 26.0, 424 (two and one) 41.1 and 28.0, 541
+// (two each) 43.8 and 47.9, 1,082 (four and three) 89.4 and 78.7, 2,990
+// (17,939 triangles x 40 bands) 247 and 200. 1 in FP32 (2 there: 0.136 -> 0.149
+// ms on the triangles). The FP32 form is at 64 registers, four blocks per SM: the
 // constants of the end are formed at the start for it (at 72, with three
 // blocks, 147 us on the triangles instead of 135).
 constexpr int kMomSlots = 12;
@@ -4150,8 +4152,19 @@ void Solver::launch_moments(S *eps, bool apply, int d0, int nbt, bool accumulate
                                                                     Tlat_, E_, q_, Tband_, Th_, Q_, apply ? 1 : 0, d0,
                                                                     nbt, accumulate ? 1 : 0);
     };
-    if constexpr (sizeof(S) == 8)
-        if (nb % 2 == 0 && grid >= 148) return go(std::integral_constant<int, 2>{});
+    if constexpr (sizeof(S) == 8) {
+        if (nb % 2 == 0 && moments_bands_ == 0) {
+            // waves of the launch with one and with two bands per thread
+            int sms = 0, fit[2] = {0, 0};
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit[0], k_moments<S, 1>, (cpb * nb + 31) / 32 * 32, moments_smem());
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit[1], k_moments<S, 2>, (cpb * (nb / 2) + 31) / 32 * 32,
+                                                          moments_smem());
+            auto waves = [&](int f) { return (grid + f * sms - 1) / std::max(1, f * sms); };
+            moments_bands_ = fit[0] > 0 && fit[1] > 0 && waves(fit[1]) < waves(fit[0]) ? 2 : 1;
+        }
+        if (nb % 2 == 0 && moments_bands_ == 2) return go(std::integral_constant<int, 2>{});
+    }
     go(std::integral_constant<int, 1>{});
 }
 

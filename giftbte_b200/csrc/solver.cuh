@@ -216,6 +216,7 @@ public:
     bool face_path() const;
     void launch_walls(bool moments);
     size_t moments_smem() const;
+    int moments_bands_ = 0;  // bands per thread of the FP64 moments (0: not yet chosen)
     template <typename S> void launch_moments(S *eps, bool apply, int d0, int nbt, bool accumulate);
     int tuned_res_form_ = 0;     // residual launch shape (1 thread per cell, 5/6 warp per cell; 0 = not yet tuned)
     int last_res_form_ = 0;      // the same, of the last solve's residual launches (0: 1-band form)
