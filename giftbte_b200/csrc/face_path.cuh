@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(256, 3) k_tr_step_face(DMesh m, DPhys p, int c
 // k_bound_out with the gradients of the wall cells only (gw of k_grad_face):
 // e_c(new) + g_c(pre-sweep) . (x_f - x_c) on the walls a direction leaves. A
 // thread per (wall side, band) walks its block's share of the directions
-// (wall_grid): 0.30 -> 0.14 ms against a thread per value (4,800 wall faces x
+// (dir_grid): 0.30 -> 0.14 ms against a thread per value (4,800 wall faces x
 // 40 bands x 128 directions).
 template <typename S, int DIM>
 __global__ void __launch_bounds__(256) k_bound_out_w(DMesh m, DPhys p, const S *__restrict__ eps,
@@ -523,9 +523,9 @@ __global__ void __launch_bounds__(256) k_bound_out_w(DMesh m, DPhys p, const S *
     const double nx = m.cf_nx[k], ny = m.cf_ny[k], nz = m.cf_nz[k];
     const double rx = m.cf_fx[k] - m.cx[c], ry = m.cf_fy[k] - m.cy[c], rz = m.cf_fz[k] - m.cz[c];
     const double gx = gTb[3 * c], gy = gTb[3 * c + 1], gz = gTb[3 * c + 2];
-    const int per = (ndb + gridDim.y - 1) / gridDim.y, d1 = min((int)(blockIdx.y + 1) * per, ndb);
+    const DirRange r = dir_share(ndb);
 #pragma unroll 4
-    for (int dl = blockIdx.y * per; dl < d1; dl++) {
+    for (int dl = r.first; dl < r.end; dl++) {
         const int d = d0 + dl;
         const double vn = vm * p.sx[d] * nx + vm * p.sy[d] * ny + vm * p.sz[d] * nz;
         if (!(vn >= 0)) continue;

@@ -84,25 +84,29 @@ int grid_for(size_t total, int threads = kThreads) {
     return (int)std::max<size_t>(1, std::min<size_t>(g, 148 * 64));
 }
 
-// a thread per item, kDirShare directions each
+// A thread per item and share of the directions: at most kDirShare each, and as
+// few (2 at least) as it takes to give every SM four blocks. The kernel takes
+// its share from the grid. (240 wall faces x 20 bands x 32 directions, outgoing
+// values: one thread for all of them 19.4 us, now 6.9.)
 constexpr int kDirShare = 32;
 dim3 dir_grid(size_t items, int nd) {
-    return dim3((unsigned)((items + kThreads - 1) / kThreads), (nd + kDirShare - 1) / kDirShare);
+    const unsigned gx = (unsigned)((items + kThreads - 1) / kThreads);
+    const unsigned want = std::max((unsigned)((nd + kDirShare - 1) / kDirShare), (4 * 148 + gx - 1) / gx);
+    return dim3(gx, std::min(want, (unsigned)(nd + 1) / 2));
 }
-// the same with as few directions per thread (2 at least) as it takes to give
-// every SM four blocks; the kernel takes its share from the grid (240 wall
-// faces x 20 bands x 32 directions: one thread for all of them 19.4 us, now 6.9)
-dim3 wall_grid(size_t items, int nd) {
-    const int gx = (int)((items + kThreads - 1) / kThreads);
-    const int want = std::max((nd + kDirShare - 1) / kDirShare, (4 * 148 + gx - 1) / gx);
-    return dim3(gx, std::min(want, (nd + 1) / 2));
+struct DirRange {
+    int first, end;
+};
+__device__ __forceinline__ DirRange dir_share(int nd) {
+    const int per = (nd + gridDim.y - 1) / gridDim.y;
+    return {min((int)blockIdx.y * per, nd), min((int)(blockIdx.y + 1) * per, nd)};
 }
 
 // ---------------------------------------------------------------- kernels --
 
 // The passes that set up the stored deviations and their base. Each owns what
 // does not depend on the direction (a cell's band, a cell's faces) and walks
-// kDirShare directions, so the cell's index arithmetic, constants
+// its share of the directions (dir_grid), so the cell's index arithmetic, constants
 // and FP64 face geometry are formed once for all of them; bound by the HBM
 // traffic of the band state. 48,000 tetrahedra x 40 bands x 128 directions
 // (FP32), against a thread per value: init 0.64 -> 0.15 ms, rebase 0.77 ->
@@ -116,8 +120,8 @@ __global__ void __launch_bounds__(256) k_init_eps(DMesh m, DPhys p, const double
     const int b = (int)(t % p.nb), c = (int)(t / p.nb);
     const int mo = mat_off(p, c);
     const S v = (S)(p.C[mo + b] * T0[c] - p.C[mo + b] * Tb[c]);
-    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, p.nd);
-    for (int d = blockIdx.y * kDirShare; d < d1; d++) eps[d * row + t] = v;
+    const DirRange r = dir_share(p.nd);
+    for (int d = r.first; d < r.end; d++) eps[d * row + t] = v;
 }
 
 // eps += C_b (Tb_old - Tb_new): moves the base of the stored deviation to a
@@ -129,9 +133,9 @@ __global__ void __launch_bounds__(256) k_rebase(DMesh m, DPhys p, const double *
     if (t >= row) return;
     const int b = (int)(t % p.nb), c = (int)(t / p.nb);
     const double Cb = p.C[mat_off(p, c) + b], dT = Tb_old[c] - Tb_new[c];
-    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, p.nd);
+    const DirRange r = dir_share(p.nd);
 #pragma unroll 8
-    for (int d = blockIdx.y * kDirShare; d < d1; d++) eps[d * row + t] = (S)((double)eps[d * row + t] + Cb * dT);
+    for (int d = r.first; d < r.end; d++) eps[d * row + t] = (S)((double)eps[d * row + t] + Cb * dT);
 }
 
 // least-squares gradient of a cell field with the same stencil. ROUND_EACH:
@@ -605,8 +609,8 @@ __global__ void __launch_bounds__(256) k_base_flux(DMesh m, DPhys p, const doubl
             if (DIM == 3) in[f] += gTb[3 * j + 2] * (m.cf_fz[k] - m.cz[j]);
         }
     }
-    const int d1 = min((int)(blockIdx.y + 1) * kDirShare, p.nd);
-    for (int d = blockIdx.y * kDirShare; d < d1; d++) {
+    const DirRange r = dir_share(p.nd);
+    for (int d = r.first; d < r.end; d++) {
         const double sx = p.sx[d], sy = p.sy[d], sz = p.sz[d];
         double acc = 0;
 #pragma unroll
@@ -4363,7 +4367,7 @@ Error Solver::solve_t(SolveStats &st) {
             GL(K_BOUND_OUT, (k_bound_out<S, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_,
                                                                                                    d0, nbt)));
         else if (n_walls_ > 0)
-            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<wall_grid((size_t)n_walls_ * nb, nbt), kThreads, 0, s>>>(
+            GL(K_BOUND_OUT, (k_bound_out_w<S, DIM><<<dir_grid((size_t)n_walls_ * nb, nbt), kThreads, 0, s>>>(
                                 dm_, dp_, eps, (const S *)wall_grad_, n_wall_slots_, n_walls_, wall_side_, wall_slot_,
                                 Tbase_, gTb_, eb_, d0, nbt)));
     };
@@ -5123,7 +5127,7 @@ Error Solver::transient_t(double dt, double total, double err_t, double err_q, i
         if (!faces)
             k_bound_out<double, DIM><<<grid_for((size_t)nbt * nbs * nb), kThreads, 0, s>>>(dm_, dp_, ev, eb_, d0, nbt);
         else if (n_walls_ > 0)
-            k_bound_out_w<double, DIM><<<wall_grid((size_t)n_walls_ * nb, nbt), kThreads, 0, s>>>(
+            k_bound_out_w<double, DIM><<<dir_grid((size_t)n_walls_ * nb, nbt), kThreads, 0, s>>>(
                 dm_, dp_, eps, (const double *)wall_grad_, n_wall_slots_, n_walls_, wall_side_, wall_slot_, Tbase_, gTb_,
                 eb_, d0, nbt);
     };
