@@ -156,12 +156,12 @@ def kernel_algorithmic_bytes(name: str, s: int, rows: float, nb: int, nd: int, n
 # updates it processed), from ncu captures; the profiles/ summaries give the
 # commands. The 2D figures are from the full-size 17,939-cell cell.
 NCU_TRAFFIC_PER_UPDATE = {
-    ("config2", "fp32"): {"residual": 679.538432e6 / 45921280, "sweep": 389.135872e6 / 45921280,
-                          "gradient": 449.162752e6 / 45921280, "moments": 513.953024e6 / 45921280},
+    ("config2", "fp32"): {"residual": 680.424704e6 / 45923840, "sweep": 391.828480e6 / 45923840,
+                          "gradient": 455.035648e6 / 45923840, "moments": 518.938880e6 / 45923840},
     # the 3D block's figures from its h = 5 nm, 100 nm tall piece (48,000 tets,
     # 2.4576e8 updates per launch); traffic grows with the updates processed
-    ("config3", "fp32"): {"residual": 4.505939e9 / 245760000, "sweep": 2.267558e9 / 245760000,
-                          "gradient": 3.787149e9 / 245760000, "moments": 2.925927e9 / 245760000},
+    ("config3", "fp32"): {"residual": 4.504945e9 / 245760000, "sweep": 2.268682e9 / 245760000,
+                          "gradient": 3.794071e9 / 245760000, "moments": 2.930045e9 / 245760000},
 }
 
 

@@ -114,10 +114,12 @@ __device__ __forceinline__ void lds(unsigned a, FaceW<double, 3> &t) {
 // for the outgoing wall values that follow the sweep, its gradient to
 // gw[batch direction][wall slot][DIM][band] for each of its wall faces.
 //
-// Bound by the shared-memory pipe: a row load serves 128 bands of a stencil
-// entry in four wavefronts, the entry itself costs about two and a half
-// however few cells share it. Several pieces per lane (NP) share the entry;
-// in 3D the slab they need would leave one CTA per SM, so NP = 1 there.
+// What bounds it are the shared loads and the staging: a row load serves 128
+// bands of a stencil entry in four wavefronts, the entry itself costs about two
+// and a half however few cells share it. Several pieces per lane (NP) share the
+// entry; in 3D the slab they need would leave one CTA per SM, so NP = 1 there.
+// In 3D the pipe is 64% busy and a quarter of the warps are there to cover the
+// loads' latency and the next slab's copies; in 2D it is 70% busy.
 // Writing face values instead of gradients leaves its time where the tiled
 // gradient's was (17,939 triangles x 40 x 64 FP32: 0.23 -> 0.25 ms; 48,000
 // tetrahedra x 40 x 128 FP32: 4.85 -> 4.85 ms; 12,000 FP64: 3.18 -> 2.85 ms);

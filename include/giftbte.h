@@ -194,8 +194,9 @@ typedef struct {
                                  form, band count a multiple of 32, 40 or 48; others run 2);
                                  0 = automatic: with residual_form 0 the face-value kernels where
                                  they apply (second order without the limiter, band rows of whole
-                                 16-byte pieces; gbte_stats.gradient_dirs 11), else the fastest on
-                                 the first outer iteration. Results do not depend on it beyond the
+                                 16-byte pieces, no two cells that share two faces;
+                                 gbte_stats.gradient_dirs 11), else the fastest on the first
+                                 outer iteration. Results do not depend on it beyond the
                                  rounding of the operations after the gradient. */
     int residual_form;        /* launch shape of the second-order residual: 1 = a thread per cell
                                  and 4 bands, 5, 6 = a warp per cell as for gradient_dirs, 7, 8 =
