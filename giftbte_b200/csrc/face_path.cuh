@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(256, 3) k_resid_face(DMesh m, DPhys p, int cpb
 // thread that writes a value reads it, so the new field needs no second array
 // and no copy back. Bound by the face rows it streams.
 // 4,608 triangles x 20 bands x 32 directions (FP64): 27 us, and a whole step
-// 287 -> 159 us against gradient arrays, a thread per value and a copy back.
+// 287 -> 153 us against gradient arrays, a thread per value and a copy back.
 // 288 triangles x 2 bands x 256 directions: 27.6 us with eight directions each,
 // 16.6 us with four.
 template <int DIM>

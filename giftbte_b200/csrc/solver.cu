@@ -1977,8 +1977,8 @@ __global__ void k_remacro(DMesh m, const double *__restrict__ Th, const double *
 // directions: the second pass loads kWallBatch values before it stores any
 // (the compiler cannot move a load over the stores to eb), and blocks hold
 // fewer walls so that every SM has one (launch_walls): the refresh of 240 wall
-// faces x 20 bands x 32 directions 30 -> 19 us. Where a block would still have
-// few threads and many directions (few bands), the directions are split.
+// faces x 20 bands x 32 directions 30 -> 19 us. Where a block still has room for
+// more threads, the directions are split: 11 us.
 constexpr int kWallSlots = 8, kWallBatch = 8;
 template <bool MOM>
 __global__ void __launch_bounds__(256) k_walls(DMesh m, DPhys p, int cpb, int split, int nw,
