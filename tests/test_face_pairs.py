@@ -16,7 +16,7 @@ EXE = os.path.join(ROOT, "giftbte_b200", "_build", "tests", "face_pairs")
 
 
 @pytest.fixture(scope="module")
-def checker():
+def driver():
     os.makedirs(os.path.dirname(EXE), exist_ok=True)
     srcs = [os.path.join(ROOT, "tests", "cpp", "face_pairs_main.cpp")] + [
         os.path.join(CSRC, f) for f in ("mesh.cpp", "angles.cpp", "deck.cpp")]
@@ -31,9 +31,9 @@ def checker():
     (lambda: make_golden.load("quad_heat_specular")[0], 1),
     (lambda: decks.config3_deck(h_nm=25.0, size_nm=(50.0, 50.0, 50.0), n_bands=2), 1),
 ], ids=["notched", "square", "interface", "quads", "block"])
-def test_paired_faces_and_centres(checker, tmp_path, make, paired):
+def test_paired_faces_and_centres(driver, tmp_path, make, paired):
     make().write(str(tmp_path))
-    r = subprocess.run([checker, str(tmp_path)], capture_output=True, text=True)
+    r = subprocess.run([driver, str(tmp_path)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     f = dict(zip(r.stdout.split()[0::2], r.stdout.split()[1::2]))
     assert int(f["paired"]) == paired

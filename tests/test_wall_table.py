@@ -15,7 +15,7 @@ EXE = os.path.join(ROOT, "giftbte_b200", "_build", "tests", "wall_check")
 
 
 @pytest.fixture(scope="module")
-def checker():
+def driver():
     os.makedirs(os.path.dirname(EXE), exist_ok=True)
     srcs = [os.path.join(ROOT, "tests", "cpp", "wall_check_main.cpp")] + [
         os.path.join(CSRC, f) for f in ("mesh.cpp", "angles.cpp", "deck.cpp")]
@@ -29,9 +29,9 @@ def checker():
     (lambda: twice(decks.config1_deck(6), [1, 3]), 24, 36),
     (lambda: decks.config3_deck(h_nm=25.0, size_nm=(50.0, 50.0, 50.0), n_bands=2), 48, 48),
 ], ids=["square", "interface", "twice", "block"])
-def test_table_and_its_check(checker, tmp_path, make, slots, walls):
+def test_table_and_its_check(driver, tmp_path, make, slots, walls):
     make().write(str(tmp_path))
-    r = subprocess.run([checker, str(tmp_path)], capture_output=True, text=True)
+    r = subprocess.run([driver, str(tmp_path)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
     last = r.stdout.split("\n")[-2].split()
     assert (int(last[1]), int(last[3])) == (slots, walls)
